@@ -9,6 +9,8 @@
 // sgd.rs:210), GradScaler::unscale_ (ferrotorch-optim/src/grad_scaler.rs:200-240), HAS_INF_NAN (kernels.rs:6205).
 #include "common.cuh"
 #include "host_common.h"
+#include <algorithm>
+#include <vector>
 
 namespace {
 
@@ -315,6 +317,185 @@ FT_EXPORT int ft_sgd_flat(float* master, void* p_bf16, float* buf, const void* g
   else
     sgd_kernel<float><<<grid, 256, 0, st>>>(master, (__nv_bfloat16*)p_bf16, buf, (const float*)grad, (size_t)n, a, grad_scale_ptr);
   return (int)cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------------------------------------
+// One launch for the parameter tensors of a whole model.
+//
+// A model's list holds a few large weights among many vectors (ResNet-50: 161 tensors, two thirds of them below 2048 elements), for which a launch
+// per tensor costs more than the update: 161 launches took 2.6 ms of host time for 0.56 ms of kernels. The table of addresses travels as a kernel
+// parameter (48 bytes an entry, so nothing is copied to the device and the launch can be captured); the work is cut into chunks of
+// MULTI_CHUNK elements, which the CTAs of one wave take in turn: a chunk finds its tensor by bisection over the running chunk counts, seven uniform
+// loads from the constant bank. The arithmetic is that of the flat kernels. A chunk whose addresses are not all 16-byte aligned is walked
+// element by element. Bound by DRAM where the tensors are large: 28 bytes an element for AdamW.
+// Measured: AdamW.step over 161 f32 tensors, 22 M elements together: 2628 us with a launch per tensor, 368 us now, of which the walk over the list in Python is most.
+// ---------------------------------------------------------------------------------------------------------
+namespace {
+constexpr int MULTI_MAX = 128, MULTI_CHUNK = 4096;
+struct MultiEntry { float* w; __nv_bfloat16* low; float* s0; float* s1; const void* grad; int64_t n; };
+struct MultiTable {
+  int count;
+  unsigned first[MULTI_MAX + 1];       // first[i]: chunks ahead of tensor i
+  MultiEntry e[MULTI_MAX];
+};
+
+struct AdamWOp {
+  AdamWArgs a;
+  FT_DEVICE void operator()(float& p, float& m, float& v, float g) const {
+    const float decay = 1.f - a.lr * a.weight_decay, step = a.lr / a.bias_c1, inv_c2 = rsqrtf(a.bias_c2);
+    if (a.maximize) g = -g;
+    p *= decay;
+    m = a.beta1 * m + (1.f - a.beta1) * g;
+    v = a.beta2 * v + (1.f - a.beta2) * g * g;
+    const float denom = sqrtf(v) * inv_c2 + a.eps;
+    p -= step * m / denom;
+  }
+};
+
+struct SgdOp {
+  SgdArgs a;
+  FT_DEVICE void operator()(float& p, float& buf, float&, float g) const {
+    if (a.maximize) g = -g;
+    if (a.weight_decay != 0.f) g += a.weight_decay * p;
+    if (a.momentum != 0.f) {
+      const float b = a.first_step ? g : a.momentum * buf + (1.f - a.dampening) * g;
+      buf = b;
+      g = a.nesterov ? g + a.momentum * b : b;
+    }
+    p -= a.lr * g;
+  }
+};
+
+FT_DEVICE float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+FT_DEVICE float4 load4(const __nv_bfloat16* p) {
+  const uint2 raw = *reinterpret_cast<const uint2*>(p);
+  const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+
+template <typename GradT, typename Op>
+__global__ void __launch_bounds__(256) multi_update_kernel(const __grid_constant__ MultiTable t, const Op op) {
+  const unsigned chunks = t.first[t.count];
+  for (unsigned c = blockIdx.x; c < chunks; c += gridDim.x) {
+    int lo = 0, hi = t.count - 1;                       // the last tensor with first[lo] <= c
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (t.first[mid] <= c) lo = mid; else hi = mid - 1;
+    }
+    const MultiEntry& e = t.e[lo];
+    const int64_t at = (int64_t)(c - t.first[lo]) * MULTI_CHUNK;
+    const int n = (int)min((int64_t)MULTI_CHUNK, e.n - at);
+    float* w = e.w + at;
+    float* s0 = e.s0 ? e.s0 + at : nullptr;
+    float* s1 = e.s1 ? e.s1 + at : nullptr;
+    __nv_bfloat16* low = e.low ? e.low + at : nullptr;
+    const GradT* grad = static_cast<const GradT*>(e.grad) + at;
+    const bool wide = ((reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(s0) | reinterpret_cast<uintptr_t>(s1) | reinterpret_cast<uintptr_t>(low) |
+                        reinterpret_cast<uintptr_t>(grad)) & 15) == 0;
+    int i = threadIdx.x * 4;
+    if (wide) {
+      for (; i + 4 <= n; i += 1024) {
+        const float4 g4 = load4(grad + i), p4 = load4(w + i);
+        const float4 a4 = s0 ? load4(s0 + i) : make_float4(0.f, 0.f, 0.f, 0.f), b4 = s1 ? load4(s1 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float p[4] = {p4.x, p4.y, p4.z, p4.w}, a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
+        const float g[4] = {g4.x, g4.y, g4.z, g4.w};
+#pragma unroll
+        for (int k = 0; k < 4; k++) op(p[k], a[k], b[k], g[k]);
+        *reinterpret_cast<float4*>(w + i) = make_float4(p[0], p[1], p[2], p[3]);
+        if (s0) *reinterpret_cast<float4*>(s0 + i) = make_float4(a[0], a[1], a[2], a[3]);
+        if (s1) *reinterpret_cast<float4*>(s1 + i) = make_float4(b[0], b[1], b[2], b[3]);
+        if (low) {
+          const __nv_bfloat162 h0 = __floats2bfloat162_rn(p[0], p[1]), h1 = __floats2bfloat162_rn(p[2], p[3]);
+          *reinterpret_cast<uint2*>(low + i) = make_uint2(*reinterpret_cast<const uint32_t*>(&h0), *reinterpret_cast<const uint32_t*>(&h1));
+        }
+      }
+    }
+    // what is left: the last n % 4 elements, or all of an unaligned chunk
+    for (int k = (wide ? (n & ~3) : 0) + threadIdx.x; k < n; k += 256) {
+      float p = w[k], a = s0 ? s0[k] : 0.f, b = s1 ? s1[k] : 0.f;
+      op(p, a, b, (float)grad[k]);
+      w[k] = p;
+      if (s0) s0[k] = a;
+      if (s1) s1[k] = b;
+      if (low) low[k] = __float2bfloat16(p);
+    }
+  }
+}
+
+// Whether no launch over these tensors could write what another of its chunks reads or writes: their address ranges are disjoint where one is written.
+bool multi_disjoint(const int64_t* rows, int count, int grad_bytes) {
+  struct Range { uint64_t at, end; bool written; };
+  std::vector<Range> r;
+  r.reserve((size_t)count * 5);
+  for (int i = 0; i < count; i++) {
+    const int64_t* t = rows + 6 * i;
+    const int bytes[5] = {4, 2, 4, 4, grad_bytes};
+    for (int k = 0; k < 5; k++)
+      if (t[k]) r.push_back({(uint64_t)t[k], (uint64_t)t[k] + (uint64_t)t[5] * bytes[k], k != 4});
+  }
+  std::sort(r.begin(), r.end(), [](const Range& a, const Range& b) { return a.at < b.at; });
+  uint64_t end = 0, end_written = 0;
+  for (const Range& x : r) {
+    if (x.at < end_written || (x.written && x.at < end)) return false;
+    end = std::max(end, x.end);
+    if (x.written) end_written = std::max(end_written, x.end);
+  }
+  return true;
+}
+
+template <typename GradT, typename Op>
+int multi_update(const int64_t* rows, int count, Op op, cudaStream_t st) {
+  if (count <= 0) return FT_ERR_ARG;
+  for (int i = 0; i < count; i++)
+    if (rows[6 * i + 5] <= 0 || !rows[6 * i] || !rows[6 * i + 4]) return FT_ERR_ARG;
+  static int resident = 0;
+  if (!resident) {
+    int r = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, multi_update_kernel<GradT, Op>, 256, 0) != cudaSuccess || r < 1) r = 4;
+    cudaGetLastError();
+    resident = r;
+  }
+  // tensors that share memory are updated one after another, in the order of the list
+  const int most = multi_disjoint(rows, count, (int)sizeof(GradT)) ? MULTI_MAX : 1;
+  MultiTable t;
+  for (int i = 0; i < count;) {
+    uint64_t chunks = 0;
+    t.count = 0;
+    for (; i < count && t.count < most; i++) {
+      const int64_t* row = rows + 6 * i;
+      const uint64_t mine = ((uint64_t)row[5] + MULTI_CHUNK - 1) / MULTI_CHUNK;
+      if (mine > 0x7fffffffull) return FT_ERR_TOO_LARGE;
+      if (t.count && chunks + mine > 0x7fffffffull) break;
+      t.first[t.count] = (unsigned)chunks;
+      t.e[t.count++] = {(float*)row[0], (__nv_bfloat16*)row[1], (float*)row[2], (float*)row[3], (const void*)row[4], row[5]};
+      chunks += mine;
+    }
+    t.first[t.count] = (unsigned)chunks;
+    const int grid = (int)std::min<uint64_t>(chunks, 148ull * resident);
+    multi_update_kernel<GradT, Op><<<grid, 256, 0, st>>>(t, op);
+    FT_CUDA_TRY(cudaGetLastError());
+  }
+  return FT_OK;
+}
+}  // namespace
+
+// AdamW over `count` tensors: rows of six 64-bit values on the host, [master f32, bf16 copy or 0, first moment, second moment, gradient, elements]. All tensors
+// are at the same step and their gradients have one type (grad_dtype: 0 = bf16, 1 = f32).
+FT_EXPORT int ft_adamw_multi(const int64_t* rows, int count, int grad_dtype, float lr, float beta1, float beta2, float eps, float weight_decay, int step, int maximize,
+                             cudaStream_t st) {
+  if (step < 1) return FT_ERR_ARG;
+  const AdamWOp op{{lr, beta1, beta2, eps, weight_decay, 1.f - powf(beta1, (float)step), 1.f - powf(beta2, (float)step), maximize}};
+  return grad_dtype == 0 ? multi_update<__nv_bfloat16>(rows, count, op, st) : multi_update<float>(rows, count, op, st);
+}
+
+// SGD over `count` tensors: rows [master f32, bf16 copy or 0, momentum buffer or 0, 0, gradient, elements].
+FT_EXPORT int ft_sgd_multi(const int64_t* rows, int count, int grad_dtype, float lr, float momentum, float dampening, float weight_decay, int nesterov, int first_step,
+                           int maximize, cudaStream_t st) {
+  if (momentum != 0.f)
+    for (int i = 0; i < count; i++)
+      if (!rows[6 * i + 2]) return FT_ERR_ARG;
+  const SgdOp op{{lr, momentum, dampening, weight_decay, nesterov, first_step, maximize}};
+  return grad_dtype == 0 ? multi_update<__nv_bfloat16>(rows, count, op, st) : multi_update<float>(rows, count, op, st);
 }
 
 // Squared L2 norm of a flat buffer into *total_sq (device). `partial` is scratch of >= 1184 floats.

@@ -6,6 +6,8 @@ GradScaler::unscale_ (ferrotorch-optim/src/grad_scaler.rs:200-240).
 """
 from __future__ import annotations
 
+import array
+
 import torch
 
 from .. import _lib
@@ -58,6 +60,39 @@ def sgd_flat_(master: torch.Tensor, p_bf16: torch.Tensor | None, buf: torch.Tens
     master.add_(g, alpha=-lr)
     if p_bf16 is not None:
         p_bf16.copy_(master)
+
+
+class MultiUpdate:
+    """Collects the tensors of one optimizer step and updates them with a launch per kind (gradient type, step or first step) instead of one per tensor, when the block
+    ends. The tensors are held until :meth:`flush`, which launches on the stream that is current then."""
+
+    def __init__(self, launcher: str, hyper, maximize: bool):
+        self.launcher, self.hyper, self.maximize = launcher, hyper, int(maximize)
+        self.rows: dict = {}
+        self.held: list = []
+
+    def __enter__(self) -> "MultiUpdate":
+        return self
+
+    def __exit__(self, *exc) -> None:
+        self.flush()
+
+    def add(self, kind, master, low, s0, s1, grad) -> None:
+        """``kind``: the step of AdamW, whether the step is the first of SGD."""
+        key = (grad.dtype is torch.float32, kind)
+        rows = self.rows.get(key)
+        if rows is None:
+            rows = self.rows[key] = []
+        rows += (master.data_ptr(), 0 if low is None else low.data_ptr(), 0 if s0 is None else s0.data_ptr(), 0 if s1 is None else s1.data_ptr(), grad.data_ptr(),
+                 grad.numel())
+        self.held.append((master, low, s0, s1, grad))
+
+    def flush(self) -> None:
+        rows, self.rows = self.rows, {}
+        for (f32, kind), values in rows.items():
+            table = array.array("q", values)
+            _lib.call(self.launcher, _lib.c_void_p(table.buffer_info()[0]), len(values) // 6, int(f32), *self.hyper, int(kind), self.maximize, _lib.S())
+        self.held.clear()
 
 
 def grad_norm_(buffers, max_norm: float = 0.0, found_inf: torch.Tensor | None = None):

@@ -17,6 +17,7 @@ import torch
 from .. import ops
 from ..errors import InvalidArgument
 from ..nn.compute_copy import mark_synced, optimizer_target
+from ..ops.optim import MultiUpdate
 
 
 class _Cfg:
@@ -131,48 +132,58 @@ class Sgd(Optimizer):
             with torch.enable_grad():
                 loss = closure()
         for g in self.param_groups:
-            for p in g["params"]:
-                if p.grad is None:
-                    continue
-                st = self.state[p]
-                first = "buf" not in st
-                target = optimizer_target(p) if p.dtype == torch.float32 else None
-                if _fused_ok(p, p.grad) or (target is not None and _flat_pair_ok(p, p.grad, need_cuda=False)):
-                    grad = p.grad
-                    if not (p.is_contiguous() and grad.is_contiguous()) and grad.stride() != p.stride():
-                        grad = torch.empty_like(p, dtype=grad.dtype).copy_(grad)      # bring the gradient into the parameter's memory order
-                    if first:
-                        st["buf"] = torch.zeros(p.numel(), device=p.device, dtype=torch.float32) if g["momentum"] else None
-                        if p.dtype == torch.bfloat16:
-                            st["master"] = _flat(p.detach()).float().clone()
-                    layout = None if p.is_contiguous() else p.stride()          # None: row-major order
-                    if not first and st.get("layout") != layout and st["buf"] is not None:
-                        # the parameter was re-laid-out since the last step: re-order the momentum buffer to match
-                        old_stride = st.get("layout") or torch.empty(p.shape, device="meta").stride()
-                        old = torch.as_strided(st["buf"], p.shape, old_stride)
-                        st["buf"] = _flat(torch.empty_like(p, dtype=torch.float32).copy_(old)).clone()
-                    st["layout"] = layout
-                    master = st.get("master", _flat(p.detach()))
-                    low = _flat(p.detach()) if p.dtype == torch.bfloat16 else (_flat(target) if target is not None else None)
-                    ops.sgd_flat_(master, low, st["buf"], _flat(grad), lr=g["lr"],
-                                  momentum=g["momentum"], dampening=g["dampening"], weight_decay=g["weight_decay"], nesterov=g["nesterov"],
-                                  first_step=first, maximize=g["maximize"])
+            with MultiUpdate("ft_sgd_multi", (g["lr"], g["momentum"], g["dampening"], g["weight_decay"], int(g["nesterov"])), g["maximize"]) as many:
+                self._step_group(g, many)
+        return loss
+
+    def _step_group(self, g, many) -> None:
+        for p in g["params"]:
+            if p.grad is None:
+                continue
+            st = self.state[p]
+            first = "buf" not in st
+            target = optimizer_target(p) if p.dtype == torch.float32 else None
+            if _fused_ok(p, p.grad) or (target is not None and _flat_pair_ok(p, p.grad, need_cuda=False)):
+                grad = p.grad
+                if not (p.is_contiguous() and grad.is_contiguous()) and grad.stride() != p.stride():
+                    grad = torch.empty_like(p, dtype=grad.dtype).copy_(grad)      # bring the gradient into the parameter's memory order
+                if first:
+                    st["buf"] = torch.zeros(p.numel(), device=p.device, dtype=torch.float32) if g["momentum"] else None
+                    if p.dtype == torch.bfloat16:
+                        st["master"] = _flat(p.detach()).float().clone()
+                layout = None if p.is_contiguous() else p.stride()          # None: row-major order
+                if not first and st.get("layout") != layout and st["buf"] is not None:
+                    # the parameter was re-laid-out since the last step: re-order the momentum buffer to match
+                    old_stride = st.get("layout") or torch.empty(p.shape, device="meta").stride()
+                    old = torch.as_strided(st["buf"], p.shape, old_stride)
+                    st["buf"] = _flat(torch.empty_like(p, dtype=torch.float32).copy_(old)).clone()
+                st["layout"] = layout
+                master = st.get("master", _flat(p.detach()))
+                low = _flat(p.detach()) if p.dtype == torch.bfloat16 else (_flat(target) if target is not None else None)
+                if p.is_cuda and p.numel():
+                    many.add(first, master, low, st["buf"], None, _flat(grad))
                     if target is not None:
                         mark_synced(p)
                     continue
-                d = -p.grad if g["maximize"] else p.grad
-                if g["weight_decay"]:
-                    d = d.add(p, alpha=g["weight_decay"])
-                if g["momentum"]:
-                    if first:
-                        st["buf"] = d.clone()
-                    else:
-                        st["buf"].mul_(g["momentum"]).add_(d, alpha=1 - g["dampening"])
-                    d = d.add(st["buf"], alpha=g["momentum"]) if g["nesterov"] else st["buf"]
-                elif first:
-                    st["buf"] = None
-                p.add_(d, alpha=-g["lr"])
-        return loss
+                ops.sgd_flat_(master, low, st["buf"], _flat(grad), lr=g["lr"],
+                              momentum=g["momentum"], dampening=g["dampening"], weight_decay=g["weight_decay"], nesterov=g["nesterov"],
+                              first_step=first, maximize=g["maximize"])
+                if target is not None:
+                    mark_synced(p)
+                continue
+            many.flush()                                                  # updates stay in the order of the list
+            d = -p.grad if g["maximize"] else p.grad
+            if g["weight_decay"]:
+                d = d.add(p, alpha=g["weight_decay"])
+            if g["momentum"]:
+                if first:
+                    st["buf"] = d.clone()
+                else:
+                    st["buf"].mul_(g["momentum"]).add_(d, alpha=1 - g["dampening"])
+                d = d.add(st["buf"], alpha=g["momentum"]) if g["nesterov"] else st["buf"]
+            elif first:
+                st["buf"] = None
+            p.add_(d, alpha=-g["lr"])
 
 
 class AdamW(Optimizer):
@@ -194,55 +205,66 @@ class AdamW(Optimizer):
                 loss = closure()
         for g in self.param_groups:
             b1, b2 = g["betas"]
-            for p in g["params"]:
-                if p.grad is None:
-                    continue
-                st = self.state[p]
-                if not st:
-                    st["step"] = 0
-                    st["exp_avg"] = torch.zeros(p.numel(), device=p.device, dtype=torch.float32)
-                    st["exp_avg_sq"] = torch.zeros(p.numel(), device=p.device, dtype=torch.float32)
-                    if g["amsgrad"]:
-                        st["max_exp_avg_sq"] = torch.zeros(p.numel(), device=p.device, dtype=torch.float32)
-                    if p.dtype != torch.float32:
-                        st["master"] = p.detach().float().reshape(-1).clone()
-                st["step"] += 1
-                t = st["step"]
-                grad = p.grad
-                # a row-major f32 parameter with a compute copy takes the flat kernel on any device: the copy is rewritten with the master
-                target = optimizer_target(p) if (p.dtype == torch.float32 and p.is_contiguous() and grad.is_contiguous()) else None
-                if self._decoupled and not g["amsgrad"] and (_fused_ok(p, grad) or (target is not None and not grad.is_sparse)):
-                    master = st.get("master", p.view(-1))
-                    low = p.view(-1) if p.dtype == torch.bfloat16 else (target.view(-1) if target is not None else None)
-                    ops.adamw_flat_(master, low, st["exp_avg"], st["exp_avg_sq"],
-                                    grad.reshape(-1), lr=g["lr"], beta1=b1, beta2=b2, eps=g["eps"], weight_decay=g["weight_decay"], step=t,
-                                    maximize=g["maximize"])
+            with MultiUpdate("ft_adamw_multi", (g["lr"], b1, b2, g["eps"], g["weight_decay"]), g["maximize"]) as many:
+                self._step_group(g, b1, b2, many)
+        return loss
+
+    def _step_group(self, g, b1, b2, many) -> None:
+        for p in g["params"]:
+            if p.grad is None:
+                continue
+            st = self.state[p]
+            if not st:
+                st["step"] = 0
+                st["exp_avg"] = torch.zeros(p.numel(), device=p.device, dtype=torch.float32)
+                st["exp_avg_sq"] = torch.zeros(p.numel(), device=p.device, dtype=torch.float32)
+                if g["amsgrad"]:
+                    st["max_exp_avg_sq"] = torch.zeros(p.numel(), device=p.device, dtype=torch.float32)
+                if p.dtype != torch.float32:
+                    st["master"] = p.detach().float().reshape(-1).clone()
+            st["step"] += 1
+            t = st["step"]
+            grad = p.grad
+            # a row-major f32 parameter with a compute copy takes the flat kernel on any device: the copy is rewritten with the master
+            target = optimizer_target(p) if (p.dtype == torch.float32 and p.is_contiguous() and grad.is_contiguous()) else None
+            if self._decoupled and not g["amsgrad"] and (_fused_ok(p, grad) or (target is not None and not grad.is_sparse)):
+                master = st.get("master", p)
+                low = p if p.dtype == torch.bfloat16 else target
+                if p.is_cuda and p.numel():
+                    many.add(t, master, low, st["exp_avg"], st["exp_avg_sq"], grad)
                     if target is not None:
                         mark_synced(p)
                     continue
-                gr = grad.detach().float().reshape(-1)
-                if g["maximize"]:
-                    gr = -gr
-                master = st.get("master", None)
-                # moments and gradient are walked in logical (row-major) order; an f32 parameter whose memory is not row-major (the
-                # convolution weights of a channels-last model) is updated through a row-major copy that is written back below
-                writeback = master is None and not p.is_contiguous()
-                w = master if master is not None else (p.detach().reshape(-1).clone() if writeback else p.view(-1))
-                if self._decoupled:
-                    w.mul_(1 - g["lr"] * g["weight_decay"])
-                elif g["weight_decay"]:
-                    gr = gr.add(w, alpha=g["weight_decay"])                    # coupled L2 (Adam)
-                st["exp_avg"].mul_(b1).add_(gr, alpha=1 - b1)
-                st["exp_avg_sq"].mul_(b2).addcmul_(gr, gr, value=1 - b2)
-                c1, c2 = 1 - b1 ** t, 1 - b2 ** t
-                v = st["exp_avg_sq"]
-                if g["amsgrad"]:
-                    torch.maximum(st["max_exp_avg_sq"], v, out=st["max_exp_avg_sq"])
-                    v = st["max_exp_avg_sq"]
-                w.addcdiv_(st["exp_avg"], (v.sqrt() / math.sqrt(c2)).add_(g["eps"]), value=-g["lr"] / c1)
-                if master is not None or writeback:
-                    p.copy_(w.view_as(p))
-        return loss
+                master, low = master.view(-1), None if low is None else low.view(-1)
+                ops.adamw_flat_(master, low, st["exp_avg"], st["exp_avg_sq"],
+                                grad.reshape(-1), lr=g["lr"], beta1=b1, beta2=b2, eps=g["eps"], weight_decay=g["weight_decay"], step=t,
+                                maximize=g["maximize"])
+                if target is not None:
+                    mark_synced(p)
+                continue
+            many.flush()                                                  # updates stay in the order of the list
+            gr = grad.detach().float().reshape(-1)
+            if g["maximize"]:
+                gr = -gr
+            master = st.get("master", None)
+            # moments and gradient are walked in logical (row-major) order; an f32 parameter whose memory is not row-major (the
+            # convolution weights of a channels-last model) is updated through a row-major copy that is written back below
+            writeback = master is None and not p.is_contiguous()
+            w = master if master is not None else (p.detach().reshape(-1).clone() if writeback else p.view(-1))
+            if self._decoupled:
+                w.mul_(1 - g["lr"] * g["weight_decay"])
+            elif g["weight_decay"]:
+                gr = gr.add(w, alpha=g["weight_decay"])                    # coupled L2 (Adam)
+            st["exp_avg"].mul_(b1).add_(gr, alpha=1 - b1)
+            st["exp_avg_sq"].mul_(b2).addcmul_(gr, gr, value=1 - b2)
+            c1, c2 = 1 - b1 ** t, 1 - b2 ** t
+            v = st["exp_avg_sq"]
+            if g["amsgrad"]:
+                torch.maximum(st["max_exp_avg_sq"], v, out=st["max_exp_avg_sq"])
+                v = st["max_exp_avg_sq"]
+            w.addcdiv_(st["exp_avg"], (v.sqrt() / math.sqrt(c2)).add_(g["eps"]), value=-g["lr"] / c1)
+            if master is not None or writeback:
+                p.copy_(w.view_as(p))
 
 
 class Adam(AdamW):

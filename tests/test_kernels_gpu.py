@@ -173,6 +173,38 @@ def test_sgd_flat_matches_torch():
     assert (master - ref.detach()).abs().max().item() < 1e-5
 
 
+@pytest.mark.parametrize("rule", ["adamw", "sgd"])
+@pytest.mark.parametrize("gdtype", [torch.float32, torch.bfloat16])
+def test_multi_update_matches_flat(rule, gdtype):
+    """A list of tensors in one launch gives what a launch per tensor gives: sizes around a chunk (4096) and a vector (4), more tensors than one table holds (128),
+    addresses that are not 16-byte aligned, a tensor that appears twice (updated twice, one after the other)."""
+    from ferrotorch_b200.ops.optim import MultiUpdate
+    sizes = [1, 3, 4, 5, 4095, 4096, 4097, 8191, 70001] + list(range(1, 130))
+    rows = []
+    for n in sizes:
+        off = n % 3 if n > 100 else 0
+        make = lambda dt=torch.float32: torch.randn(n + 4, device="cuda").to(dt)[off: off + n]        # noqa: E731
+        rows.append([make(), make(torch.bfloat16) if n % 2 else None, make(), make().abs(), make(gdtype)])
+    want = [[t if t is None else t.clone() for t in r] for r in rows]
+    many = MultiUpdate(*(("ft_adamw_multi", (1e-2, 0.9, 0.95, 1e-8, 0.1)) if rule == "adamw" else ("ft_sgd_multi", (0.1, 0.9, 0.0, 1e-4, 1))), False)
+    order = list(range(len(rows)))
+    for repeat in (order, [8, 8, 5]):
+        with many:
+            for i in repeat:
+                many.add(3 if rule == "adamw" else False, *rows[i][:3], rows[i][3] if rule == "adamw" else None, rows[i][4])
+        for i in repeat:
+            w, low, s0, s1, g = want[i]
+            if rule == "adamw":
+                ops.adamw_flat_(w, low, s0, s1, g, lr=1e-2, beta1=0.9, beta2=0.95, eps=1e-8, weight_decay=0.1, step=3)
+            else:
+                ops.sgd_flat_(w, low, s0, g, lr=0.1, momentum=0.9, weight_decay=1e-4, nesterov=True)
+    for got, exp in zip(rows, want):
+        for a, b in zip(got, exp):
+            if a is not None:
+                # the compiler may contract other pairs of the same operations: a few roundings of 2^-24 of values below ten; a 16-bit copy may then round the other way
+                torch.testing.assert_close(a.float(), b.float(), rtol=2e-6 if a.dtype == torch.float32 else 2.0 ** -7, atol=2e-6)
+
+
 def test_grad_norm_and_scale():
     torch.manual_seed(9)
     a = torch.randn(100003, device="cuda")
