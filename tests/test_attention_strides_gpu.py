@@ -1,0 +1,61 @@
+"""Attention on operands read where they lie: head sizes around the kernels' 64 and 128 columns, lengths around their blocks, layouts that tile loads take and layouts that need a
+copy, groups of query heads shared by a cluster; values and gradients against the f32 materialised form."""
+import pytest
+import torch
+
+import ferrotorch_b200.nn as nn
+
+pytestmark = pytest.mark.gpu
+
+# bf16 operands and probabilities carry 2^-9 relative error each; sums over keys average it: 2 % of the norm bounds forward and backward
+TOL = 2e-2
+
+
+def _layout(kind, B, H, S, D):
+    if kind == "heads":                                     # contiguous [B, H, S, D]
+        return torch.randn(B, H, S, D, device="cuda").bfloat16()
+    if kind == "rows":                                      # a projection's [B, S, H * D]
+        return torch.randn(B, S, H * D, device="cuda").bfloat16().view(B, S, H, D).transpose(1, 2)
+    if kind == "slice":                                     # columns of a wider row
+        return torch.randn(B, S, H, D + 8, device="cuda").bfloat16()[..., 8:].transpose(1, 2)
+    if kind == "odd":                                       # rows off the 16-byte boundaries
+        return torch.randn(B, H, S, D + 1, device="cuda").bfloat16()[..., 1:]
+    if kind == "shared":                                    # one head seen as all of them
+        return torch.randn(B, 1, S, D, device="cuda").bfloat16().expand(B, H, S, D)
+    return torch.randn(B, H, D, S, device="cuda").bfloat16().transpose(2, 3)
+
+
+@pytest.mark.parametrize("kinds", [("heads", "rows", "slice"), ("rows", "odd", "columns"), ("slice", "shared", "heads")])
+@pytest.mark.parametrize("B,Hq,Hkv,S,D,causal", [(1, 1, 1, 1, 8, True), (2, 3, 1, 63, 64, True), (1, 4, 2, 64, 72, False), (2, 2, 2, 65, 56, False), (1, 4, 1, 127, 128, True),
+                                                 (3, 4, 4, 129, 64, True), (1, 8, 2, 193, 80, True), (1, 8, 1, 640, 128, True), (1, 6, 3, 257, 32, False)])
+def test_strided_attention(B, Hq, Hkv, S, D, causal, kinds):
+    if ops_backend() != "tcgen05":
+        pytest.skip("native attention kernels not built")
+    torch.manual_seed(S + D)
+    q, k, v = (_layout(kind, B, h, S, D).requires_grad_() for kind, h in zip(kinds, (Hq, Hkv, Hkv)))
+    qf, kf, vf = (t.detach().double().requires_grad_() for t in (q, k, v))
+    o = nn.functional.scaled_dot_product_attention(q, k, v, is_causal=causal)
+    ref = nn.standard_attention(qf, nn.repeat_kv(kf, Hq // Hkv), nn.repeat_kv(vf, Hq // Hkv), causal)
+    g = torch.randn(B, S, Hq, D, device="cuda").bfloat16().transpose(1, 2)
+    got, want = torch.autograd.grad(o, (q, k, v), g), torch.autograd.grad(ref, (qf, kf, vf), g.double())
+    assert o.shape == (B, Hq, S, D)
+    assert (o.double() - ref).norm() <= TOL * ref.norm()
+    # single keys: the gradients of q and k are sums of differences that cancel, so their error is measured against the gradient's scale without cancellation
+    floor = 1e-2 * g.double().norm() if S > 1 else 0.1 * g.double().norm()
+    for a, b in zip(got, want):
+        assert a.shape == b.shape and (a.double() - b).norm() <= TOL * b.norm() + 2e-2 * floor
+
+
+def ops_backend():
+    from ferrotorch_b200 import ops
+    return ops.attention.backend()
+
+
+@pytest.mark.parametrize("refused", ["batch", "heads", "device"])
+def test_operands_that_do_not_fit_are_refused(refused):
+    q = torch.zeros(2, 4, 16, 64, device="cuda", dtype=torch.bfloat16)
+    k = v = torch.zeros(1 if refused == "batch" else 2, 2, 16, 64, device="cpu" if refused == "device" else "cuda", dtype=torch.bfloat16)
+    if refused == "heads":
+        v = torch.zeros(2, 4, 16, 64, device="cuda", dtype=torch.bfloat16)
+    with pytest.raises(Exception):
+        nn.functional.scaled_dot_product_attention(q, k, v)
