@@ -9,6 +9,7 @@ dependency on the driver.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 import re
@@ -101,8 +102,23 @@ def ptr(t) -> int:
     return 0 if t is None else t.data_ptr()
 
 
+_raw_stream, _get_device = getattr(torch._C, "_cuda_getCurrentRawStream", None), getattr(torch._C, "_cuda_getDevice", None)
+_in_place = contextlib.nullcontext()
+
+
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream of the current device. Asked of the runtime directly once CUDA is up: going through a Stream object takes several microseconds, on
+    every launch."""
+    if _raw_stream is None or not torch.cuda.is_initialized():
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_get_device())
+
+
+def on_device_of(t):
+    """A context in which the device of ``t`` is the current one; nothing is entered where it already is."""
+    if _get_device is not None and t.device.index == _get_device():
+        return _in_place
+    return torch.cuda.device(t.device)
 
 
 # Argument signatures of the exported launchers are read from the sources themselves
@@ -155,6 +171,9 @@ def _fn(fn_name: str):
     return f
 
 
+_PLAIN = frozenset((int, float, bool, type(None)))
+
+
 def _unwrap(a):
     if isinstance(a, torch.Tensor):
         return a.data_ptr()
@@ -195,11 +214,11 @@ def call(fn_name: str, *args) -> None:
     Tensors are passed as their data pointers, ``None`` as a null pointer.
     """
     global launch_calls
-    fn = _fn(fn_name)
+    fn = _bound.get(fn_name) or _fn(fn_name)
     launch_calls += 1
     if len(args) != len(fn.argtypes):
         raise FerrotorchError(f"{fn_name}: expected {len(fn.argtypes)} arguments, got {len(args)}")
-    raw = [_unwrap(a) for a in args]
+    raw = [a if type(a) in _PLAIN else _unwrap(a) for a in args]
     if _trace is None:
         check(fn(*raw), fn_name)
         return
@@ -222,9 +241,4 @@ def read_status() -> int:
     return out.value
 
 
-def P(t):
-    return c_void_p(ptr(t))
-
-
-def S():
-    return c_void_p(stream_ptr())
+P, S = ptr, stream_ptr          # short forms for the arguments of :func:`call`

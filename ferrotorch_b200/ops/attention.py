@@ -164,7 +164,7 @@ class _HeadsFn(torch.autograd.Function):
         (q_, sq), (k_, sk), (v_, sv) = _readable(q), _readable(k), _readable(v)
         out = torch.empty((B, S, Hq, D), device=q.device, dtype=q.dtype)
         lse = torch.empty((B, Hq, S), device=q.device, dtype=torch.float32)
-        with torch.cuda.device(q.device):
+        with _lib.on_device_of(q):
             _launch_fwd(((q_.data_ptr(), sq), (k_.data_ptr(), sk), (v_.data_ptr(), sv)), out.data_ptr(), lse, B, S, Hq, Hkv, D, (S * Hq * D, D, Hq * D), causal, scale)
         ctx.save_for_backward(q, k, v, out, lse)
         ctx.causal, ctx.scale = causal, scale
@@ -183,7 +183,7 @@ class _HeadsFn(torch.autograd.Function):
         (q_, sq), (k_, sk), (v_, sv), (o_, so), (do_, sdo) = (_readable(t) for t in (q, k, v, out, dout))
         grads = [torch.empty((B, S, h, D), device=q.device, dtype=q.dtype) for h in (Hq, Hkv, Hkv)]
         rows = [(t.data_ptr(), (S * h * D, D, h * D)) for t, h in zip(grads, (Hq, Hkv, Hkv))]
-        with torch.cuda.device(q.device):
+        with _lib.on_device_of(q):
             _launch_bwd(((q_.data_ptr(), sq), (k_.data_ptr(), sk), (v_.data_ptr(), sv)), (o_.data_ptr(), so), lse, (do_.data_ptr(), sdo), rows, B, S, Hq, Hkv, D,
                         ctx.causal, ctx.scale)
         return (*(t.transpose(1, 2) for t in grads), None, None)

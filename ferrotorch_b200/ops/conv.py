@@ -79,7 +79,7 @@ def _wgrad_rows(a_rows: torch.Tensor, b_rows: torch.Tensor, shifts) -> torch.Ten
         planes = _plane_cache(a_rows.device, splits * n_out)[: splits * n_out]
         out = torch.empty((Co, 9, C), device=a_rows.device, dtype=torch.float32)
         arr = (ctypes.c_int * 9)(*[int(v) for v in shifts])
-        with torch.cuda.device(a_rows.device):
+        with _lib.on_device_of(a_rows):
             _lib.call("ft_conv_wgrad_shift_splitk", a_rows, b_rows, planes, Co, C, J, R, arr, splits, _lib.S())
             _lib.call("ft_splitk_reduce", planes, splits, Co, 9 * C, ctypes.c_int64(9 * C), ctypes.c_int64(n_out), None, out,
                       ctypes.c_int64(9 * C), 1, _lib.S())
@@ -128,7 +128,7 @@ def _rows_gemm(x_rows: torch.Tensor, w: torch.Tensor, rows: int, shifts, bias=No
         y = torch.empty((rows, Cout), device=x_rows.device, dtype=torch.bfloat16)
         arr = (ctypes.c_int * taps)(*[int(v) for v in shifts])
         b = None if bias is None else bias.to(torch.bfloat16).contiguous()
-        with torch.cuda.device(x_rows.device):
+        with _lib.on_device_of(x_rows):
             _lib.call("ft_conv_rows_gemm", x_rows, w.contiguous(), y, b, rows, R, Cin, Cout, taps, arr, 1 if relu else 0, _lib.S())
         return y
     acc = torch.zeros(rows, Cout)
@@ -272,7 +272,7 @@ def conv3x3_nhwc_raw(x: torch.Tensor, w_krsc: torch.Tensor, relu: bool = False) 
             y = torch.relu(y)
         return y.to(torch.bfloat16).contiguous(memory_format=torch.channels_last)
     y = torch.empty((N, Cout, H, W), device=x.device, dtype=torch.bfloat16, memory_format=torch.channels_last)
-    with torch.cuda.device(x.device):
+    with _lib.on_device_of(x):
         _lib.call("ft_conv3x3_nhwc", x, w_krsc, y, N, H, W, Cin, Cout, int(relu), _lib.S())
     return y
 

@@ -105,14 +105,14 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
         if not gated:
             gate.wait(b)
     if gated:
-        with torch.cuda.device(a.device):
+        with _lib.on_device_of(a):
             _lib.call("ft_gemm_gated", _lib.P(a), _lib.P(b), _lib.P(out), M, N, K, ctypes.c_int64(a.stride(0)), ctypes.c_int64(b.stride(0)),
                       ctypes.c_int64(out.stride(0)), int(a_mn), int(b_mn), int(out_dtype == torch.float32), ctypes.c_void_p(gate.counters_ptr),
                       gate.expected, ctypes.c_void_p(gate.slot_ptr), ctypes.c_int64(gate.piece_bytes), _lib.S())
         gate.mark(b)
         return out
     if in_f16 or act is not None and _ACT[act] or residual is not None:
-        with torch.cuda.device(a.device):
+        with _lib.on_device_of(a):
             _lib.call("ft_gemm_ex", _lib.P(a), _lib.P(b), _lib.P(out), _lib.P(bias), _lib.P(residual), M, N, K, ctypes.c_int64(a.stride(0)), ctypes.c_int64(b.stride(0)),
                       ctypes.c_int64(out.stride(0)), ctypes.c_int64(residual.stride(0) if residual is not None else 0), int(a_mn), int(b_mn),
                       int(out_dtype == torch.float32), int(in_f16), _ACT[act], _lib.S())
@@ -121,13 +121,13 @@ def gemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = F
     if splits > 1:
         # few output tiles and a long K (weight gradients of 1x1 convolutions, decode): spread K over the SMs as f32 planes, then sum
         planes = _plane_cache(a.device, splits * M * N)[: splits * M * N].view(splits, M, N)
-        with torch.cuda.device(a.device):
+        with _lib.on_device_of(a):
             _lib.call("ft_gemm_bf16_splitk", _lib.P(a), _lib.P(b), _lib.P(planes), M, N, K, ctypes.c_int64(a.stride(0)), ctypes.c_int64(b.stride(0)),
                       ctypes.c_int64(N), int(a_mn), int(b_mn), splits, _lib.S())
             _lib.call("ft_splitk_reduce", _lib.P(planes), splits, M, N, ctypes.c_int64(N), ctypes.c_int64(M * N), _lib.P(bias), _lib.P(out),
                       ctypes.c_int64(out.stride(0)), int(out_dtype == torch.float32), _lib.S())
         return out
-    with torch.cuda.device(a.device):
+    with _lib.on_device_of(a):
         _lib.call("ft_gemm_bf16", _lib.P(a), _lib.P(b), _lib.P(out), _lib.P(bias), M, N, K, ctypes.c_int64(a.stride(0)),
                   ctypes.c_int64(b.stride(0)), ctypes.c_int64(out.stride(0)), int(a_mn), int(b_mn),
                   int(out_dtype == torch.float32), _lib.S())

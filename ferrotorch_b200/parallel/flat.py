@@ -36,6 +36,14 @@ class TensorSpec:
             n *= s
         return n
 
+    @property
+    def stride(self) -> Tuple[int, ...]:
+        """Row-major."""
+        out = [1] * len(self.shape)
+        for i in range(len(self.shape) - 2, -1, -1):
+            out[i] = out[i + 1] * self.shape[i + 1]
+        return tuple(out)
+
 
 def _round_up(x: int, m: int) -> int:
     return (x + m - 1) // m * m
@@ -53,6 +61,7 @@ class FlatUnit:
         for n, shp in shapes:
             self.specs[n] = TensorSpec(n, off, tuple(shp))
             off = _round_up(off + self.specs[n].numel, align)
+        self._layout = [(n, s.shape, s.stride, s.offset) for n, s in self.specs.items()]
         self.numel = off
         self.padded = _round_up(off, world * align)
         self.chunk = self.padded // world
@@ -87,7 +96,11 @@ class FlatUnit:
         return b[s.offset: s.offset + s.numel].view(s.shape)
 
     def views(self, buf: torch.Tensor | None = None) -> Dict[str, torch.Tensor]:
-        return {n: self.view(n, buf) for n in self.specs}
+        b = self.full if buf is None else buf
+        if b.requires_grad or b.dim() != 1 or b.stride(0) != 1 or b.numel() < self.numel:
+            return {n: self.view(n, b) for n in self.specs}
+        at = b.storage_offset()                       # one view each instead of a slice and a view: a layer asks for its views three times a step
+        return {n: b.as_strided(shape, stride, at + offset) for n, shape, stride, offset in self._layout}
 
     def shard_slice(self, buf: torch.Tensor, rank: int | None = None) -> torch.Tensor:
         r = self.rank if rank is None else rank
