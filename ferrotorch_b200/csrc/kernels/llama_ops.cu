@@ -136,29 +136,102 @@ __global__ void embedding_bwd_kernel(const int64_t* __restrict__ ids, const __nv
   }
 }
 
-// Deterministic form: the token rows are visited grouped by id (the caller sorted the ids stably and passes the permutation and the segment
-// bounds), one CTA per distinct id, each output element summed in f32 in token order by one thread. No atomics: the same bits on every run.
+// Deterministic forms: each output element is summed in f32 in token order by one thread, no atomics: the same bits on every run. One CTA per token and 8 columns per
+// thread; the CTA of an id's first token adds all its rows to the table, the others have nothing to do.
+FT_DEVICE void add_row(float (&acc)[8], const __nv_bfloat16* row) {
+  float f[8];
+  bf16x8_to_float(*reinterpret_cast<const bf16x8*>(row), f);
+#pragma unroll
+  for (int e = 0; e < 8; e++) acc[e] += f[e];
+}
 template <typename AccT>
-__global__ void __launch_bounds__(128) embedding_bwd_sorted_kernel(const int64_t* __restrict__ uniq_ids, const int64_t* __restrict__ seg_end,
-                                                                   const int64_t* __restrict__ perm, const __nv_bfloat16* __restrict__ dout,
-                                                                   AccT* __restrict__ dtable, int n_uniq, int d, int64_t vocab) {
-  for (int u = blockIdx.x; u < n_uniq; u += gridDim.x) {
-    const int64_t id = uniq_ids[u];
-    if (id < 0 || id >= vocab) continue;
-    const int64_t k0 = u == 0 ? 0 : seg_end[u - 1], k1 = seg_end[u];
-    for (int c = threadIdx.x * 8; c < d; c += blockDim.x * 8) {
-      float acc[8];
+FT_DEVICE void load_sum(float (&acc)[8], const AccT* at) {        // the running sum that is already in the table
 #pragma unroll
-      for (int e = 0; e < 8; e++) acc[e] = (float)dtable[(size_t)id * d + c + e];        // running sum already in the table
-      for (int64_t k = k0; k < k1; k++) {
-        float f[8];
-        bf16x8_to_float(*reinterpret_cast<const bf16x8*>(dout + (size_t)perm[k] * d + c), f);
+  for (int e = 0; e < 8; e++) acc[e] = (float)at[e];
+}
+template <typename AccT>
+FT_DEVICE void store_sum(const float (&acc)[8], AccT* at) {
 #pragma unroll
-        for (int e = 0; e < 8; e++) acc[e] += f[e];
-      }
-#pragma unroll
-      for (int e = 0; e < 8; e++) dtable[(size_t)id * d + c + e] = (AccT)acc[e];
+  for (int e = 0; e < 8; e++) at[e] = (AccT)acc[e];
+}
+
+// The ids as they come: every CTA looks through all of them for its own. tokens^2 comparisons out of L2, which for up to SCAN_TOKENS tokens takes less than
+// sorting them first (a sort of 4096 ids alone takes 40 us in one CTA, and is five launches); nothing goes through the host.
+// Against the sort, the run lengths and their copy to the host before: 2331 tokens of width 1024 55 us in eight launches and a wait of the host -> 15 us in one;
+// 128 tokens of width 256 23 -> 4 us.
+constexpr int SCAN_TOKENS = 4096;
+template <typename AccT>
+__global__ void __launch_bounds__(512) embedding_bwd_scan_kernel(const int64_t* __restrict__ ids, const __nv_bfloat16* __restrict__ dout, AccT* __restrict__ dtable,
+                                                                 int tokens, int d, int64_t vocab) {
+  __shared__ uint16_t found[SCAN_TOKENS];
+  __shared__ int counts[17];
+  const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  const int64_t id = ids[t];
+  if (id < 0 || id >= vocab) return;
+  bool before = false;
+  for (int j = threadIdx.x; j < t; j += blockDim.x) before |= ids[j] == id;
+  if (__syncthreads_or(before)) return;
+  int n = 0;                                                       // places of the id from t on, in order
+  for (int j0 = t; j0 < tokens; j0 += blockDim.x) {
+    const int j = j0 + threadIdx.x;
+    const bool mine = j < tokens && ids[j] == id;
+    if (!__syncthreads_or(mine)) continue;
+    const unsigned in_warp = __ballot_sync(0xffffffffu, mine);
+    if (lane == 0) counts[warp] = __popc(in_warp);
+    __syncthreads();
+    int at = n;
+    for (int w = 0; w < warps; w++) {
+      if (w < warp) at += counts[w];
+      n += counts[w];
     }
+    if (mine) found[at + __popc(in_warp & ((1u << lane) - 1))] = (uint16_t)j;
+  }
+  __syncthreads();
+  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
+  if (c >= d) return;
+  float acc[8];
+  AccT* out = dtable + (size_t)id * d + c;
+  load_sum(acc, out);
+#pragma unroll 4
+  for (int k = 0; k < n; k++) add_row(acc, dout + (size_t)found[k] * d + c);
+  store_sum(acc, out);
+}
+
+// The ids sorted stably, with the permutation that sorted them: the first place of a run adds the run.
+template <typename AccT>
+__global__ void __launch_bounds__(512) embedding_bwd_runs_kernel(const int64_t* __restrict__ sorted_ids, const int64_t* __restrict__ perm,
+                                                                 const __nv_bfloat16* __restrict__ dout, AccT* __restrict__ dtable, int tokens, int d, int64_t vocab) {
+  const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
+  const int t = blockIdx.x;
+  const int64_t id = sorted_ids[t];
+  if (id < 0 || id >= vocab || c >= d || (t > 0 && sorted_ids[t - 1] == id)) return;
+  float acc[8];
+  AccT* out = dtable + (size_t)id * d + c;
+  load_sum(acc, out);
+  for (int k = t; k < tokens && sorted_ids[k] == id; k++) add_row(acc, dout + (size_t)perm[k] * d + c);
+  store_sum(acc, out);
+}
+
+// out = x * g and table *= g in place, g a bf16-rounded scalar in device memory: what a loss's gradient does to the gradients that its forward pass prepared for 1.
+// A factor of 1 (every step of a training loop) leaves the table alone; it is seen here and not on the host, which does not wait for it.
+__global__ void __launch_bounds__(256) scale_grads_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ out, size_t n, __nv_bfloat16* __restrict__ table,
+                                                          size_t n_table, const float* __restrict__ g) {
+  const float f = __bfloat162float(__float2bfloat16(*g));
+  const size_t first = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+  for (size_t i = first; i < n; i += step) {
+    float v[8];
+    bf16x8_to_float(reinterpret_cast<const bf16x8*>(x)[i], v);
+#pragma unroll
+    for (int e = 0; e < 8; e++) v[e] *= f;
+    reinterpret_cast<bf16x8*>(out)[i] = float_to_bf16x8(v);
+  }
+  if (f == 1.f) return;
+  for (size_t i = first; i < n_table; i += step) {
+    float v[8];
+    bf16x8_to_float(reinterpret_cast<const bf16x8*>(table)[i], v);
+#pragma unroll
+    for (int e = 0; e < 8; e++) v[e] *= f;
+    reinterpret_cast<bf16x8*>(table)[i] = float_to_bf16x8(v);
   }
 }
 
@@ -231,16 +304,30 @@ FT_EXPORT int ft_embedding_bwd(const int64_t* ids, const void* dout, void* dtabl
   return (int)cudaGetLastError();
 }
 
-// uniq_ids [n_uniq]: the distinct ids in ascending order; seg_end [n_uniq]: inclusive prefix sums of their counts; perm [tokens]: token indices
-// sorted stably by id (so perm[seg_end[u-1] .. seg_end[u]) are the tokens of uniq_ids[u] in their original order). d % 8 == 0.
-FT_EXPORT int ft_embedding_bwd_sorted(const int64_t* uniq_ids, const int64_t* seg_end, const int64_t* perm, const void* dout, void* dtable, int n_uniq,
-                                      int d, int64_t vocab, int acc_f32, cudaStream_t st) {
-  if (d % 8 || n_uniq <= 0) return FT_ERR_ARG;
-  const int grid = n_uniq < 148 * 16 ? n_uniq : 148 * 16;
-  if (acc_f32)
-    embedding_bwd_sorted_kernel<float><<<grid, 128, 0, st>>>(uniq_ids, seg_end, perm, (const __nv_bfloat16*)dout, (float*)dtable, n_uniq, d, vocab);
-  else
-    embedding_bwd_sorted_kernel<__nv_bfloat16><<<grid, 128, 0, st>>>(uniq_ids, seg_end, perm, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dtable, n_uniq, d, vocab);
+// Most tokens that ft_embedding_bwd_by_id takes in their own order.
+FT_EXPORT int ft_embedding_bwd_scan_max() { return SCAN_TOKENS; }
+
+// dtable[ids[t], :] += dout[t, :] without atomics. perm null: ids in token order, at most ft_embedding_bwd_scan_max() of them; otherwise ids sorted stably and the
+// permutation that sorted them. d % 8 == 0, rows on 16-byte boundaries.
+FT_EXPORT int ft_embedding_bwd_by_id(const int64_t* ids, const int64_t* perm, const void* dout, void* dtable, int tokens, int d, int64_t vocab, int acc_f32,
+                                     cudaStream_t st) {
+  if (d % 8 || tokens <= 0 || (!perm && tokens > SCAN_TOKENS)) return FT_ERR_ARG;
+  const int threads = d >= 4096 ? 512 : (d / 8 + 31) / 32 * 32;
+  const dim3 grid(tokens, (d + threads * 8 - 1) / (threads * 8));
+  const __nv_bfloat16* g = (const __nv_bfloat16*)dout;
+  if (!perm && acc_f32) embedding_bwd_scan_kernel<float><<<grid, threads, 0, st>>>(ids, g, (float*)dtable, tokens, d, vocab);
+  else if (!perm) embedding_bwd_scan_kernel<__nv_bfloat16><<<grid, threads, 0, st>>>(ids, g, (__nv_bfloat16*)dtable, tokens, d, vocab);
+  else if (acc_f32) embedding_bwd_runs_kernel<float><<<grid, threads, 0, st>>>(ids, perm, g, (float*)dtable, tokens, d, vocab);
+  else embedding_bwd_runs_kernel<__nv_bfloat16><<<grid, threads, 0, st>>>(ids, perm, g, (__nv_bfloat16*)dtable, tokens, d, vocab);
+  return (int)cudaGetLastError();
+}
+
+// out[n] = x[n] * g and table[n_table] *= g, bf16, with the f32 scalar *g rounded to bf16. n % 8 == n_table % 8 == 0, 16-byte aligned.
+FT_EXPORT int ft_scale_grads(const void* x, void* out, int64_t n, void* table, int64_t n_table, const float* g, cudaStream_t st) {
+  if (n % 8 || n_table % 8 || n < 0 || n_table < 0 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(table)) & 15))
+    return FT_ERR_ARG;
+  scale_grads_kernel<<<grid_for((size_t)(n > n_table / 8 ? n : n_table / 8) / 8, 256), 256, 0, st>>>((const __nv_bfloat16*)x, (__nv_bfloat16*)out, (size_t)n / 8,
+                                                                                                    (__nv_bfloat16*)table, (size_t)n_table / 8, g);
   return (int)cudaGetLastError();
 }
 

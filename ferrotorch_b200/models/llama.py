@@ -269,10 +269,8 @@ class _LMHeadLossFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         (dh,) = ctx.saved_tensors
-        # the engine calls backward with g == 1; a different upstream scale is folded into both gradients here
-        if not (g.numel() == 1 and float(g) == 1.0):
-            dh = dh * g.to(dh.dtype)
-            ctx.owner.acquire_grads()["weight"].mul_(g.to(dh.dtype))
+        # the gradients were computed for g == 1; another upstream scale is folded into both of them here, on the device
+        dh = ops.scale_grads(dh, ctx.owner.acquire_grads()["weight"], g)
         ctx.owner.grads_ready()
         return dh, None, None, None, None, None
 

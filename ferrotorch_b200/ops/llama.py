@@ -176,19 +176,28 @@ def embedding_fwd(ids: torch.Tensor, table: torch.Tensor) -> torch.Tensor:
     return table[flat].reshape(*ids.shape, table.shape[1])
 
 
+def scale_grads(x: torch.Tensor, table: torch.Tensor, g: torch.Tensor) -> torch.Tensor:
+    """``x * g`` as a new tensor, and ``table *= g`` in place, for a one-element ``g`` rounded to their type first."""
+    if (x.is_cuda and x.dtype == table.dtype == torch.bfloat16 and g.dtype == torch.float32 and g.is_cuda and x.is_contiguous() and table.is_contiguous()
+            and x.numel() % 8 == table.numel() % 8 == 0 and x.data_ptr() % 16 == table.data_ptr() % 16 == 0):
+        out = torch.empty_like(x)
+        _lib.call("ft_scale_grads", x, out, x.numel(), table, table.numel(), g, _lib.S())
+        return out
+    table.mul_(g.to(table.dtype))
+    return x * g.to(x.dtype)
+
+
 def embedding_bwd(ids: torch.Tensor, dout2: torch.Tensor, dtable: torch.Tensor, deterministic: bool = True) -> torch.Tensor:
-    """``dtable[ids] += dout`` (dtable bf16 or f32, already zeroed or holding a running sum). The default groups the token rows by id (stable
-    sort) and sums each table row in token order in f32 without atomics, so repeated runs give identical bits; ``deterministic=False`` is the
+    """``dtable[ids] += dout`` (dtable bf16 or f32, already zeroed or holding a running sum). The default groups the token rows by id and sums each table row in token order in f32 without atomics, so repeated runs give identical bits; ``deterministic=False`` is the
     atomic scatter (a little faster, order of the additions left to the hardware)."""
     flat = ids.reshape(-1).contiguous()
     if dtable.is_cuda and dout2.dtype == torch.bfloat16:
         d = dtable.shape[1]
-        if deterministic and d % 8 == 0:
-            sorted_ids, perm = torch.sort(flat, stable=True)
-            uniq, counts = torch.unique_consecutive(sorted_ids, return_counts=True)
-            seg_end = torch.cumsum(counts, 0)
-            _lib.call("ft_embedding_bwd_sorted", uniq, seg_end, perm, dout2, dtable, uniq.numel(), d, dtable.shape[0],
-                      int(dtable.dtype == torch.float32), _lib.S())
+        if deterministic and d % 8 == 0 and flat.numel():
+            perm = None
+            if flat.numel() > _lib.kernels().ft_embedding_bwd_scan_max():
+                flat, perm = torch.sort(flat, stable=True)
+            _lib.call("ft_embedding_bwd_by_id", flat, perm, dout2, dtable, flat.numel(), d, dtable.shape[0], int(dtable.dtype == torch.float32), _lib.S())
             return dtable
         _lib.call("ft_embedding_bwd", flat, dout2, dtable, flat.numel(), d, dtable.shape[0],
                   int(dtable.dtype == torch.float32), _lib.S())

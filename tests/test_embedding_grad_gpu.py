@@ -1,0 +1,42 @@
+"""Gradient of the embedding table by id, in token order, and the scaling of prepared gradients: around the number of tokens that is looked through without sorting, ids that all
+differ, repeat or lie outside the table."""
+import pytest
+import torch
+
+from ferrotorch_b200 import _lib, ops
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kind", ["random", "few", "one", "outside"])
+@pytest.mark.parametrize("tokens,d", [(1, 8), (2, 4104), (131, 256), (-1, 1032), (0, 264), (1, 520), (5000, 8)])
+def test_embedding_bwd_by_id(tokens, d, kind):
+    tokens = _lib.kernels().ft_embedding_bwd_scan_max() + tokens if tokens <= 0 or (tokens, d) == (1, 520) else tokens
+    torch.manual_seed(tokens + d)
+    vocab = 997
+    ids = torch.randint(0, {"random": vocab, "few": 3, "one": 1, "outside": vocab}[kind], (tokens,), device="cuda")
+    if kind == "outside":
+        ids[::3] = vocab
+        ids[1::5] = -1
+    dout = torch.randn(tokens, d, device="cuda").bfloat16()
+    for dtype in (torch.bfloat16, torch.float32):
+        table = torch.randn(vocab, d, device="cuda").to(dtype)
+        want = table.double()
+        ok = (ids >= 0) & (ids < vocab)
+        want.index_add_(0, ids[ok], dout[ok].double())
+        got = ops.embedding_bwd(ids, dout, table.clone())
+        # a row sums up to `tokens` terms in f32, each addition off by 2^-24 of a running sum of about sqrt(tokens); a bf16 table rounds the result once
+        bound = tokens * tokens ** 0.5 * 2 ** -23 + (2 ** -8 * want.abs() if dtype == torch.bfloat16 else 0) + 1e-6
+        assert ((got.double() - want).abs() <= bound).all()
+        assert torch.equal(got, ops.embedding_bwd(ids, dout, table.clone()))
+
+
+@pytest.mark.parametrize("g", [1.0, 0.5, 1.0001, -3.0])
+@pytest.mark.parametrize("n,m", [(8, 8), (8 * 1031, 64), (72, 8 * 70001), (12, 9)])
+def test_scale_grads(n, m, g):
+    torch.manual_seed(n)
+    x, table, f = torch.randn(n, device="cuda").bfloat16(), torch.randn(m, device="cuda").bfloat16(), torch.tensor(g, device="cuda")
+    want_x, want_t = x * f.bfloat16(), table * f.bfloat16()
+    before = x.clone()
+    out = ops.scale_grads(x, table, f)
+    assert torch.equal(out, want_x) and torch.equal(table, want_t) and torch.equal(x, before)
