@@ -85,7 +85,7 @@ def kernel_table(fn, classify, roofs, bw, fl, reps=5):
 def _by_shape(names):
     """GEMM launches by (N, K) -> label, everything else by launcher name."""
     def c(fn, raw):
-        if fn in ("ft_gemm_bf16", "ft_gemm_bf16_splitk"):
+        if fn in ("ft_gemm_bf16", "ft_gemm_bf16_splitk", "ft_gemm_stream"):
             o = 4 if fn == "ft_gemm_bf16" else 3
             return names.get((raw[o + 1], raw[o + 2]), f"gemm n={raw[o + 1]} k={raw[o + 2]}")
         if fn == "ft_gemm_grouped":

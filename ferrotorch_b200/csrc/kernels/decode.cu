@@ -27,10 +27,171 @@ constexpr int KV_BLOCK = 16;
 constexpr int MAXR = 8;
 constexpr uint64_t DEC_TIMEOUT_NS = 2000000000ull;
 
+// Sum over the planes, in their order. Eight are requested before the first is used: the planes lie in L2, and one after another each costs a round trip.
 FT_DEVICE float plane_sum(const float* __restrict__ p, int splits, size_t plane_stride, size_t idx) {
   float a = 0.f;
-  for (int s = 0; s < splits; s++) a += p[s * plane_stride + idx];
+  for (int s0 = 0; s0 < splits; s0 += 8) {
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = s0 + j < splits ? __ldcg(p + (s0 + j) * plane_stride + idx) : 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+      if (s0 + j < splits) a += v[j];
+  }
   return a;
+}
+FT_DEVICE float4 plane_sum4(const float* __restrict__ p, int splits, size_t plane_stride) {
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int s0 = 0; s0 < splits; s0 += 8) {
+    float4 v[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = s0 + j < splits ? __ldcg(reinterpret_cast<const float4*>(p + (s0 + j) * plane_stride)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+      if (s0 + j < splits) { a.x += v[j].x; a.y += v[j].y; a.z += v[j].z; a.w += v[j].w; }
+  }
+  return a;
+}
+
+// ------------------------------------------------------------------------------------------------------------
+// weight stream: P[s][t][n] = sum over a range of k of x[t][k] w[n][k], up to 16 token rows
+//
+// The product of a decode step reads every weight once, so it is bound by DRAM and, between the small kernels of a step, by how soon the stream starts. The
+// weights are the M side of the tensor-core tile (128 rows, 16 tokens: no work for padded rows, 16 accumulator columns). The (row tile, 64-wide k-block)
+// pairs are dealt to the CTAs in equal contiguous runs, so all of them end together; a tile that several CTAs share leaves one plane each, in the order of k,
+// and the CTA of its last k-block fills the planes that the tile does not need with zeros. Eleven 16 KiB stages per CTA; those of the first run are requested
+// before the wait for the previous kernel, which does not write weights: up to 24 MiB of them arrive behind the small kernels between two products.
+//
+// Before: 256-row tiles with 128 token rows, whole waves of equal K slices (up to 24 planes), loads behind the wait, one plane at a time in the kernels that read
+// them, seven launches for the end and the start of a step where there are two now. A prompt of 37 tokens and 24 steps of two layers of width 1024:
+// 4440 -> 2599 us; a prompt batch of 8 x 2048 and 32 steps of four 8B layers: 51.0 -> 46.7 ms, of which the steps are about 26 -> 21 ms.
+// ------------------------------------------------------------------------------------------------------------
+constexpr int WS_BM = 128, WS_BK = 64, WS_TOK = 16, WS_STAGES = 11, WS_THREADS = 192;
+constexpr int WS_W = WS_BM * WS_BK * 2, WS_X = WS_TOK * WS_BK * 2, WS_STAGE = WS_W + WS_X;
+constexpr int WS_SMEM = WS_STAGES * WS_STAGE + 256 + 1024;
+
+FT_DEVICE bool ws_wait(uint64_t* bar, uint32_t parity) {
+  uint64_t t0 = 0;
+  for (uint32_t i = 1;; i++) {
+    if (mbar_try_wait(bar, parity)) return true;
+    if ((i & 0xff) == 0) {
+      const uint64_t t = globaltimer_ns();
+      if (!t0) t0 = t;
+      else if (t - t0 > DEC_TIMEOUT_NS) return false;
+    }
+  }
+}
+// first (tile, k-block) pair of CTA c, and the CTA of a pair
+__host__ __device__ inline int64_t ws_first(int64_t total, int grid, int c) { return total * c / grid; }
+__host__ __device__ inline int ws_owner(int64_t total, int grid, int64_t pair) { return (int)(((pair + 1) * grid - 1) / total); }
+
+__global__ void __launch_bounds__(WS_THREADS, 1)
+gemm_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, float* __restrict__ planes, int rows, int N, int kblocks, int nplanes,
+                   int64_t ldp, uint32_t* status) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + WS_STAGES * WS_STAGE);
+  uint64_t* empty = full + WS_STAGES;
+  uint64_t* acc_full = empty + WS_STAGES;      // [2]
+  uint64_t* acc_empty = acc_full + 2;          // [2]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t total = (int64_t)((N + WS_BM - 1) / WS_BM) * kblocks;
+  const int64_t p0 = ws_first(total, gridDim.x, blockIdx.x), p1 = ws_first(total, gridDim.x, blockIdx.x + 1);
+
+  pdl_launch_dependents();
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < WS_STAGES; i++) { mbar_init(&full[i], 1); mbar_init(&empty[i], 1); }
+    for (int i = 0; i < 2; i++) { mbar_init(&acc_full[i], 1); mbar_init(&acc_empty[i], 4); }
+    mbar_fence_init();
+  }
+  if (warp == 0 && lane == 0) { tma_prefetch_desc(&tmW); tma_prefetch_desc(&tmX); }
+  if (warp == 1) { tmem_alloc(tmem_slot, 32); tmem_relinquish(); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      auto stage = [&](int s) { return smem + s * WS_STAGE; };
+      const int ahead = (int)(p1 - p0 < WS_STAGES ? p1 - p0 : WS_STAGES);
+      for (int i = 0; i < ahead; i++) {
+        mbar_expect_tx(&full[i], WS_STAGE);
+        tma_load_2d(stage(i), &tmW, &full[i], (int)((p0 + i) % kblocks) * WS_BK, (int)((p0 + i) / kblocks) * WS_BM);
+      }
+      pdl_wait();                               // the tokens come from the kernel before
+      for (int i = 0; i < ahead; i++) tma_load_2d(stage(i) + WS_W, &tmX, &full[i], (int)((p0 + i) % kblocks) * WS_BK, 0);
+      for (int64_t p = p0 + ahead; p < p1; p++) {
+        const int i = (int)(p - p0), s = i % WS_STAGES;
+        if (!ws_wait(&empty[s], ((i / WS_STAGES) & 1) ^ 1)) {
+          ft_set_status(status, FT_K_GEMM, 21, s);
+          for (int k = 0; k < 64; k++) __nanosleep(1000);           // copies in flight land before the CTA's shared memory goes away
+          break;
+        }
+        mbar_expect_tx(&full[s], WS_STAGE);
+        tma_load_2d(stage(s), &tmW, &full[s], (int)(p % kblocks) * WS_BK, (int)(p / kblocks) * WS_BM);
+        tma_load_2d(stage(s) + WS_W, &tmX, &full[s], (int)(p % kblocks) * WS_BK, 0);
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc = make_idesc_f16(WS_BM, WS_TOK, 1, 0, 0);
+      bool ok = true;
+      int seg = 0;
+      for (int64_t p = p0; p < p1 && ok; seg++) {
+        const int64_t end = min(p1, (p / kblocks + 1) * kblocks);
+        const int a = seg & 1;
+        if (!ws_wait(&acc_empty[a], ((seg >> 1) & 1) ^ 1)) { ft_set_status(status, FT_K_GEMM, 22, a); break; }
+        tc_fence_after();
+        for (bool first = true; p < end; p++, first = false) {
+          const int i = (int)(p - p0), s = i % WS_STAGES;
+          if (!ws_wait(&full[s], (i / WS_STAGES) & 1)) { ft_set_status(status, FT_K_GEMM, 23, s); ok = false; break; }
+          tc_fence_after();
+          const uint32_t w = smem_u32(smem + s * WS_STAGE), x = w + WS_W;
+#pragma unroll
+          for (int k = 0; k < WS_BK / 16; k++)
+            umma_f16_ss(tmem + a * WS_TOK, make_smem_desc(w + k * 32, 16, 1024, FT_SWZ_128B), make_smem_desc(x + k * 32, 16, 1024, FT_SWZ_128B), idesc, !(first && k == 0));
+          umma_commit(&empty[s]);
+        }
+        if (ok) umma_commit(&acc_full[a]);
+      }
+    }
+  } else {
+    pdl_wait();                                 // whoever read the planes before has finished
+    const int q = warp & 3;
+    int seg = 0;
+    for (int64_t p = p0; p < p1; seg++) {
+      const int64_t tile = p / kblocks, end = min(p1, (tile + 1) * kblocks);
+      const int a = seg & 1;
+      if (!ws_wait(&acc_full[a], (seg >> 1) & 1)) { if (lane == 0) ft_set_status(status, FT_K_GEMM, 24, a); break; }
+      tc_fence_after();
+      uint32_t v[WS_TOK];
+      tmem_ld_32x32b_x16(tmem + ((uint32_t)(q * 32) << 16) + a * WS_TOK, v);
+      tmem_ld_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[a]);
+      const int n = (int)tile * WS_BM + q * 32 + lane;
+      int plane = (int)blockIdx.x - ws_owner(total, gridDim.x, tile * kblocks);
+      if (n < N) {
+        float* out = planes + (size_t)plane * WS_TOK * ldp + n;
+#pragma unroll
+        for (int t = 0; t < WS_TOK; t++)
+          if (t < rows) out[t * ldp] = __uint_as_float(v[t]);
+        if (end == (tile + 1) * kblocks)
+          for (plane++; plane < nplanes; plane++) {
+            out = planes + (size_t)plane * WS_TOK * ldp + n;
+            for (int t = 0; t < rows; t++) out[t * ldp] = 0.f;
+          }
+      }
+      __syncwarp();
+      p = end;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem, 32); }
 }
 
 // ------------------------------------------------------------------------------------------------------------
@@ -39,8 +200,8 @@ FT_DEVICE float plane_sum(const float* __restrict__ p, int splits, size_t plane_
 template <typename OutT>
 __global__ void splitk_reduce_kernel(const float* __restrict__ partial, int splits, int rows, int N, int64_t ldp, size_t plane_stride,
                                      const __nv_bfloat16* __restrict__ bias, OutT* __restrict__ out, int64_t ldo) {
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const size_t total = (size_t)rows * N;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const int r = (int)(i / N), n = (int)(i % N);
@@ -59,8 +220,8 @@ __global__ void qkv_rope_kvwrite_kernel(const float* __restrict__ partial, int s
                                         const float* __restrict__ sin_t, __nv_bfloat16* __restrict__ q_out,
                                         __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache,
                                         const int* __restrict__ block_table, int max_blocks) {
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const int b = blockIdx.x, h = blockIdx.y, i = threadIdx.x, half = D >> 1;
   const int pos = positions[b];
   const size_t base = (size_t)b * ldp + (size_t)h * D;
@@ -140,8 +301,8 @@ __global__ void __launch_bounds__(128, 2) paged_attn_decode_kernel(const __nv_bf
                                                                 int max_blocks, const int* __restrict__ seq_lens, int Hq, int Hkv, float scale,
                                                                 float* __restrict__ ws, int* __restrict__ counters,
                                                                 __nv_bfloat16* __restrict__ out) {
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   constexpr int D = 128;
   extern __shared__ __align__(128) uint8_t pa_smem[];
   const int G = Hq / Hkv;
@@ -348,12 +509,166 @@ __global__ void __launch_bounds__(128, 2) paged_attn_decode_kernel(const __nv_bf
 }
 
 // ------------------------------------------------------------------------------------------------------------
+// ends of a decode step
+// ------------------------------------------------------------------------------------------------------------
+// x[b] = table[tokens[b]], h[b] = x[b] * rstd * w: one CTA per token, row read twice (the second time out of L1). Tokens below zero count from the table's end; one
+// outside the table reads as zeros and is reported in the status word.
+__global__ void __launch_bounds__(256) embed_norm_kernel(const int64_t* __restrict__ tokens, const __nv_bfloat16* __restrict__ table, int64_t vocab,
+                                                         const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ h, int d, float eps,
+                                                         uint32_t* status) {
+  __shared__ float red[32];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int64_t raw_id = tokens[blockIdx.x], id = raw_id < 0 ? raw_id + vocab : raw_id;
+  const bool there = id >= 0 && id < vocab;
+  if (!there && threadIdx.x == 0) ft_set_status(status, FT_K_PAGED, 31, blockIdx.x);
+  const bf16x8* src = reinterpret_cast<const bf16x8*>(table + (size_t)(there ? id : 0) * d);
+  bf16x8* xr = reinterpret_cast<bf16x8*>(x + (size_t)blockIdx.x * d);
+  bf16x8* hr = reinterpret_cast<bf16x8*>(h + (size_t)blockIdx.x * d);
+  const float keep = there ? 1.f : 0.f;
+  float ss = 0.f;
+  for (int c = threadIdx.x; c < d / 8; c += 256) {
+    float v[8];
+    bf16x8_to_float(src[c], v);
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+      v[e] = there ? v[e] : 0.f;
+      ss += v[e] * v[e];
+    }
+    xr[c] = float_to_bf16x8(v);
+  }
+  ss = block_sum(ss, red);
+  const float rstd = rsqrtf(ss / (float)d + eps) * keep;
+  for (int c = threadIdx.x; c < d / 8; c += 256) {
+    float v[8], g[8];
+    bf16x8_to_float(src[c], v);
+    bf16x8_to_float(reinterpret_cast<const bf16x8*>(w)[c], g);
+#pragma unroll
+    for (int e = 0; e < 8; e++) v[e] = there ? v[e] * rstd * g[e] : 0.f;
+    hr[c] = float_to_bf16x8(v);
+  }
+}
+
+// Order of a maximum search as an unsigned number: larger values above smaller, a NaN above all, the smaller index above the larger among equals.
+FT_DEVICE unsigned long long pick_key(float v, int i) {
+  const uint32_t u = v == 0.f ? 0u : __float_as_uint(v);            // -0 counts as 0
+  const uint32_t k = v != v ? 0xffffffffu : (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+  return (unsigned long long)k << 32 | (uint32_t)~i;
+}
+
+// The head's planes -> logits, and the place of the largest logit of every row into tokens and picked; the last CTA advances positions and lengths, so the next
+// step needs nothing from the host. best: one zero per row, done: a zero, both zero again at the end.
+__global__ void __launch_bounds__(256) logits_pick_kernel(const float* __restrict__ partial, int splits, int64_t ldp, size_t plane_stride, float* __restrict__ logits,
+                                                          int64_t ldl, int N, unsigned long long* __restrict__ best, unsigned* __restrict__ done,
+                                                          int64_t* __restrict__ tokens, int64_t* __restrict__ picked, int* __restrict__ positions, int* __restrict__ lens) {
+  __shared__ unsigned long long top[8];
+  __shared__ bool last;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int row = blockIdx.y;
+  unsigned long long mine = 0;
+  for (int c = (blockIdx.x * 256 + threadIdx.x) * 4; c < N; c += gridDim.x * 1024) {
+    float v[4];
+    if (c + 4 <= N) {
+      const float4 s = plane_sum4(partial + (size_t)row * ldp + c, splits, plane_stride);
+      v[0] = s.x; v[1] = s.y; v[2] = s.z; v[3] = s.w;
+      *reinterpret_cast<float4*>(logits + row * ldl + c) = s;
+    } else {
+      for (int e = 0; e < 4; e++) {
+        v[e] = c + e < N ? plane_sum(partial, splits, plane_stride, (size_t)row * ldp + c + e) : 0.f;
+        if (c + e < N) logits[row * ldl + c + e] = v[e];
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; e++)
+      if (c + e < N) mine = max(mine, pick_key(v[e], c + e));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mine = max(mine, __shfl_xor_sync(0xffffffffu, mine, o));
+  if ((threadIdx.x & 31) == 0) top[threadIdx.x >> 5] = mine;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int i = 1; i < 8; i++) mine = max(mine, top[i]);
+    atomicMax(best + row, mine);
+    __threadfence();
+    last = atomicAdd(done, 1u) == gridDim.x * gridDim.y - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  if (threadIdx.x < gridDim.y) {
+    const int r = threadIdx.x;
+    const int64_t at = (uint32_t)~(uint32_t)atomicExch(best + r, 0ull);
+    tokens[r] = at;
+    if (picked) picked[r] = at;
+    positions[r] += 1;
+    lens[r] += 1;
+  }
+  if (threadIdx.x == 0) *done = 0;
+}
+
+// Planes -> + residual -> RMSNorm on one rank: a row over a cluster of CTAs, its sum of squares through distributed shared memory.
+constexpr int RN_CL = 8, RN_THREADS = 128;
+__global__ void __cluster_dims__(RN_CL, 1, 1) __launch_bounds__(RN_THREADS)
+residual_norm_kernel(const float* __restrict__ partial, int splits, int64_t ldp, size_t plane_stride, __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                     __nv_bfloat16* __restrict__ h, int d, float eps) {
+  namespace cg = cooperative_groups;
+  __shared__ float red[32];
+  __shared__ float cta_ss;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int row = blockIdx.x / RN_CL, cols = ((d + RN_CL - 1) / RN_CL + 3) & ~3, c0 = (blockIdx.x % RN_CL) * cols, c1 = min(d, c0 + cols);
+  __nv_bfloat16* xr = x + (size_t)row * d;
+  pdl_launch_dependents();
+  pdl_wait();
+  float ss = 0.f;
+  for (int c = c0 + threadIdx.x * 4; c < c1; c += RN_THREADS * 4) {
+    const uint2 raw = *reinterpret_cast<const uint2*>(xr + c);
+    const float4 v = plane_sum4(partial + (size_t)row * ldp + c, splits, plane_stride);
+    const float2 x0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x)), x1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+    const __nv_bfloat162 o0 = __floats2bfloat162_rn(v.x + x0.x, v.y + x0.y), o1 = __floats2bfloat162_rn(v.z + x1.x, v.w + x1.y);
+    *reinterpret_cast<uint2*>(xr + c) = make_uint2(*reinterpret_cast<const uint32_t*>(&o0), *reinterpret_cast<const uint32_t*>(&o1));
+    const float2 f0 = __bfloat1622float2(o0), f1 = __bfloat1622float2(o1);
+    ss += f0.x * f0.x + f0.y * f0.y + f1.x * f1.x + f1.y * f1.y;
+  }
+  ss = block_sum(ss, red);
+  if (threadIdx.x == 0) cta_ss = ss;
+  cluster.sync();
+  float tot = 0.f;
+  for (int r = 0; r < RN_CL; r++) tot += *cluster.map_shared_rank(&cta_ss, r);
+  const float rstd = rsqrtf(tot / (float)d + eps);
+  for (int c = c0 + threadIdx.x * 4; c < c1; c += RN_THREADS * 4) {
+    const uint2 raw = *reinterpret_cast<const uint2*>(xr + c), wr = *reinterpret_cast<const uint2*>(w + c);
+    const float2 x0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x)), x1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+    const float2 w0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&wr.x)), w1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&wr.y));
+    const __nv_bfloat162 o0 = __floats2bfloat162_rn(x0.x * rstd * w0.x, x0.y * rstd * w0.y), o1 = __floats2bfloat162_rn(x1.x * rstd * w1.x, x1.y * rstd * w1.y);
+    *reinterpret_cast<uint2*>(h + (size_t)row * d + c) = make_uint2(*reinterpret_cast<const uint32_t*>(&o0), *reinterpret_cast<const uint32_t*>(&o1));
+  }
+  cluster.sync();                             // nobody leaves while a partner may still read its shared memory
+}
+
+// ------------------------------------------------------------------------------------------------------------
 // SwiGLU on split-K planes: P[s][b][0:F] = gate, P[s][b][F:2F] = up
 // ------------------------------------------------------------------------------------------------------------
-__global__ void decode_swiglu_kernel(const float* __restrict__ partial, int splits, int64_t ldp, size_t plane_stride, int rows, int F,
-                                     __nv_bfloat16* __restrict__ out) {
-  pdl_wait();
+// four neurons a thread
+__global__ void __launch_bounds__(128) decode_swiglu_kernel(const float* __restrict__ partial, int splits, int64_t ldp, size_t plane_stride, int rows, int F,
+                                                            __nv_bfloat16* __restrict__ out) {
   pdl_launch_dependents();
+  pdl_wait();
+  const int quads = F >> 2;
+  const size_t total = (size_t)rows * quads;
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+    const int r = (int)(i / quads), f = (int)(i % quads) * 4;
+    const float* p = partial + (size_t)r * ldp + f;
+    const float4 g = plane_sum4(p, splits, plane_stride), u = plane_sum4(p + F, splits, plane_stride);
+    auto act = [](float g, float u) { return g / (1.f + __expf(-g)) * u; };
+    const __nv_bfloat162 a = __floats2bfloat162_rn(act(g.x, u.x), act(g.y, u.y)), b = __floats2bfloat162_rn(act(g.z, u.z), act(g.w, u.w));
+    *reinterpret_cast<uint2*>(out + (size_t)r * F + f) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+  }
+}
+// neurons that do not come in fours
+__global__ void decode_swiglu_odd_kernel(const float* __restrict__ partial, int splits, int64_t ldp, size_t plane_stride, int rows, int F, __nv_bfloat16* __restrict__ out) {
+  pdl_launch_dependents();
+  pdl_wait();
   const size_t total = (size_t)rows * F;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const int r = (int)(i / F), f = (int)(i % F);
@@ -399,8 +714,8 @@ __global__ void __launch_bounds__(256) decode_ar_residual_norm_kernel(const floa
                                                                       const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ h,
                                                                       float* __restrict__ sumsq, int rows, int rows_pad, int d, int chunks, float eps,
                                                                       uint32_t* status) {
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   __shared__ float red[32];
   const int row = blockIdx.x / chunks, chunk = blockIdx.x % chunks;
   const int cols = d / chunks, c0 = chunk * cols;
@@ -466,8 +781,8 @@ decode_ar_residual_norm_cluster_kernel(const float* __restrict__ partial, int sp
                                        __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ h, int rows, int rows_pad,
                                        int d, float eps, uint32_t* status) {
   namespace cg = cooperative_groups;
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ float red[32];
   __shared__ float cta_ss;
@@ -610,8 +925,75 @@ FT_EXPORT int ft_paged_attn_decode(const void* q, const void* k_cache, const voi
 
 FT_EXPORT int ft_decode_swiglu(const float* partial, int splits, int64_t ldp, int64_t plane_stride, int rows, int F, void* out, cudaStream_t st) {
   if (rows < 1 || F < 1) return FT_ERR_ARG;
-  return (int)ft_launch_pdl(decode_swiglu_kernel, dim3(small_grid((size_t)rows * F, 256)), dim3(256), 0, st, partial, splits, ldp, (size_t)plane_stride, rows, F,
+  if (!(F & 3) && !(ldp & 3) && !(plane_stride & 3) && !((reinterpret_cast<uintptr_t>(partial) & 15) | (reinterpret_cast<uintptr_t>(out) & 7)))
+    return (int)ft_launch_pdl(decode_swiglu_kernel, dim3(small_grid((size_t)rows * F / 4, 128)), dim3(128), 0, st, partial, splits, ldp, (size_t)plane_stride, rows, F,
+                              (__nv_bfloat16*)out);
+  return (int)ft_launch_pdl(decode_swiglu_odd_kernel, dim3(small_grid((size_t)rows * F, 256)), dim3(256), 0, st, partial, splits, ldp, (size_t)plane_stride, rows, F,
                             (__nv_bfloat16*)out);
+}
+
+// How many CTAs ft_gemm_stream runs on for a weight: all, unless they would have less than four k-blocks each (a plane more costs its reader as much).
+static int ws_grid(int64_t total) { return (int)(total < 4 * 148 ? (total + 3) / 4 : 148); }
+// Number of planes that ft_gemm_stream writes for a weight [N, K].
+FT_EXPORT int ft_gemm_stream_planes(int N, int K) {
+  if (N < 1 || K < 1) return FT_ERR_ARG;
+  const int kb = (K + WS_BK - 1) / WS_BK, tiles = (N + WS_BM - 1) / WS_BM;
+  const int64_t total = (int64_t)tiles * kb;
+  const int grid = ws_grid(total);
+  int most = 1;
+  for (int t = 0; t < tiles; t++) {
+    const int n = ws_owner(total, grid, (int64_t)(t + 1) * kb - 1) - ws_owner(total, grid, (int64_t)t * kb) + 1;
+    if (n > most) most = n;
+  }
+  return most;
+}
+// planes[s][16][ldp] (f32; rows below `rows` <= 16 are written) = x[rows, K] (x) w[N, K]^T in ft_gemm_stream_planes(N, K) partial sums. bf16, K contiguous, 16-byte
+// aligned rows. w is read before the launches ahead in the stream have finished: none of them may write it.
+FT_EXPORT int ft_gemm_stream(const void* x, const void* w, float* planes, int rows, int N, int K, int64_t ldx, int64_t ldw, int64_t ldp, int nplanes, cudaStream_t st) {
+  if (rows < 1 || rows > WS_TOK || N < 1 || K < 1 || (ldx & 7) || (ldw & 7) || ldp < N || nplanes != ft_gemm_stream_planes(N, K)) return FT_ERR_ARG;
+  int dev = 0;
+  FT_CUDA_TRY(cudaGetDevice(&dev));
+  FT_CUDA_TRY(ft_bind_context(dev));
+  const int kb = (K + WS_BK - 1) / WS_BK;
+  const int64_t total = (int64_t)((N + WS_BM - 1) / WS_BM) * kb;
+  CUtensorMap tW, tX;
+  int r = ft_make_tmap_2d(&tW, w, 2, true, (uint64_t)K, (uint64_t)N, (uint64_t)ldw * 2, WS_BK, WS_BM, CU_TENSOR_MAP_SWIZZLE_128B);
+  if (r) return r;
+  r = ft_make_tmap_2d(&tX, x, 2, true, (uint64_t)K, (uint64_t)rows, (uint64_t)ldx * 2, WS_BK, WS_TOK, CU_TENSOR_MAP_SWIZZLE_128B);
+  if (r) return r;
+  static bool configured = false;
+  if (!configured) {
+    FT_CUDA_TRY(cudaFuncSetAttribute(gemm_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WS_SMEM));
+    configured = true;
+  }
+  return (int)ft_launch_pdl(gemm_stream_kernel, dim3(ws_grid(total)), dim3(WS_THREADS), (size_t)WS_SMEM, st, tW, tX, planes, rows, N, kb, nplanes, ldp, ft_status_ptr());
+}
+
+// x[b] = table[tokens[b]] (bf16 [vocab, d]), h[b] = RMSNorm(x[b]) * w. d % 8 == 0, 16-byte aligned rows.
+FT_EXPORT int ft_decode_embed_norm(const int64_t* tokens, const void* table, int64_t vocab, const void* w, void* x, void* h, int rows, int d, float eps, cudaStream_t st) {
+  if (rows < 1 || d < 8 || (d & 7) || vocab < 1) return FT_ERR_ARG;
+  return (int)ft_launch_pdl(embed_norm_kernel, dim3(rows), dim3(256), 0, st, tokens, (const __nv_bfloat16*)table, vocab, (const __nv_bfloat16*)w, (__nv_bfloat16*)x,
+                            (__nv_bfloat16*)h, d, eps, ft_status_ptr());
+}
+
+// logits[rows][ldl] = sum of the planes; tokens (and picked, if given) = place of each row's largest logit, the first of equals, a NaN before all; positions and lens
+// advance by one. ws: rows 64-bit values and one 32-bit value behind them, zeroed once. rows <= 16.
+FT_EXPORT int ft_decode_logits_pick(const float* planes, int splits, int64_t ldp, int64_t plane_stride, int rows, int N, float* logits, int64_t ldl, void* ws, int64_t* tokens,
+                                    int64_t* picked, int* positions, int* lens, cudaStream_t st) {
+  if (splits < 1 || rows < 1 || rows > WS_TOK || N < 1 || (ldp & 3) || (plane_stride & 3) || (ldl & 3) ||
+      ((reinterpret_cast<uintptr_t>(planes) | reinterpret_cast<uintptr_t>(logits)) & 15) || (reinterpret_cast<uintptr_t>(ws) & 7))
+    return FT_ERR_ARG;
+  const int need = (N + 1023) / 1024, most = 592 / rows;
+  return (int)ft_launch_pdl(logits_pick_kernel, dim3(need < most ? need : most, rows), dim3(256), 0, st, planes, splits, ldp, (size_t)plane_stride, logits, ldl, N,
+                            (unsigned long long*)ws, (unsigned*)((unsigned long long*)ws + rows), tokens, picked, positions, lens);
+}
+
+// ft_decode_ar_residual_norm for a group of one rank, without staging buffers and grid barriers. d % 4 == 0.
+FT_EXPORT int ft_decode_residual_norm(const float* partial, int splits, int64_t ldp, int64_t plane_stride, void* x, const void* w, void* h, int rows, int d, float eps,
+                                      cudaStream_t st) {
+  if (rows < 1 || splits < 1 || d < 4 || (d & 3) || (ldp & 3) || (plane_stride & 3)) return FT_ERR_ARG;
+  return (int)ft_launch_pdl(residual_norm_kernel, dim3(rows * RN_CL), dim3(RN_THREADS), 0, st, partial, splits, ldp, (size_t)plane_stride, (__nv_bfloat16*)x,
+                            (const __nv_bfloat16*)w, (__nv_bfloat16*)h, d, eps);
 }
 
 // sym_ptrs / flag_ptrs: `world` mappings of every rank's staging buffer (2 * rows_pad * d floats) and flag block (u32[8], zeroed once).

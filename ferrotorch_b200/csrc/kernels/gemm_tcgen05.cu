@@ -188,8 +188,8 @@ ft_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   // everything above touched only this CTA's shared memory and TMEM; from here on the kernel reads what its predecessor wrote
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------

@@ -396,8 +396,8 @@ __global__ void __launch_bounds__(DP_WARPS * 32) gqa_decode_prep_kernel(DecPrepA
   extern __shared__ __align__(16) float held[];      // plane sums of query and key heads: WHOLE [local unit][d16], else (halves) [warp][d16]
   __shared__ float red[32];
   __shared__ float cta_ss[2];
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const GqaDims& D = A.P.D;
   const int b = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, pos = A.P.positions[b], half = D.rot / 2, stride = gridDim.x * DP_WARPS;
   const int u0 = blockIdx.x * DP_WARPS + warp, heads = D.HQ + (cache ? D.GK : 0);
@@ -556,8 +556,8 @@ template <int NP>
 __global__ void __launch_bounds__(256) gqa_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ cache, const int* __restrict__ block_table,
                                                          int max_blocks, const int* __restrict__ seq_lens, GqaDims D, MaskGate M, int tiles, float* __restrict__ ws,
                                                          int* __restrict__ counters, Differential F, __nv_bfloat16* __restrict__ out, int64_t ldo) {
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ float sm_mx[8][GD_HT], sm_l[8][GD_HT];
   __shared__ int is_last;

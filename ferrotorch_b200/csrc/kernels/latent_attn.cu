@@ -283,8 +283,8 @@ __global__ void __launch_bounds__(PREP_THREADS) latent_decode_prep_kernel(const 
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   if (absorb) {
     const size_t qcol = (size_t)hd * (D.d8 + D.dr8);
     for (int i = threadIdx.x; i < B * D.d; i += PREP_THREADS) {
@@ -363,8 +363,8 @@ __global__ void __launch_bounds__(PREP_THREADS) latent_decode_norms_kernel(const
                                                                            const float* __restrict__ wq, const float* __restrict__ w, float eps,
                                                                            const int* __restrict__ positions, const int* __restrict__ block_table, int max_blocks,
                                                                            __nv_bfloat16* __restrict__ cq, int64_t ldq, __nv_bfloat16* __restrict__ cache) {
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(16) uint8_t prep_smem[];
   __shared__ float red[32];
   float* v = reinterpret_cast<float*>(prep_smem);
@@ -421,8 +421,8 @@ template <int MT, int NP>
 __global__ void __launch_bounds__(256, 1) latent_decode_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ cache,
                                                                const int* __restrict__ block_table, int max_blocks, const int* __restrict__ seq_lens, LatentDims D,
                                                                float scale, float* __restrict__ ws) {
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ float sm_mx[8][MT * 16], sm_l[8][MT * 16];
   constexpr int HT = MT * 16;
@@ -602,8 +602,8 @@ __global__ void __launch_bounds__(256, 1) latent_decode_kernel(const __nv_bfloat
 
 // merge the splits: grid (H, B), 128 threads; out [B][H][r16] bf16
 __global__ void __launch_bounds__(128) latent_combine_kernel(const float* __restrict__ ws, int H, int HT, int tiles, int nsplit, int r16, __nv_bfloat16* __restrict__ out) {
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   __shared__ float f[64];
   __shared__ float inv_sh;
   const int hd = blockIdx.x, b = blockIdx.y;

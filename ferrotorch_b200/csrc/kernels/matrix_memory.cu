@@ -795,8 +795,8 @@ __global__ void __launch_bounds__(256) mm_decode_kernel(MemDecode A, MemDims D, 
   float* sn = S + (size_t)D.d16 * D.v16;
   if (!zero && live && (lc % 8) == 0)
     for (int r = rg; r < D.d16; r += RG) asm volatile("prefetch.global.L2 [%0];" ::"l"(S + (size_t)r * D.v16 + col));
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const float* src = A.planes + (size_t)b * A.ldp;
   const float scale = rsqrtf((float)D.d), m_old = zero ? 0.f : sn[D.d16];
   for (int i = tid; i < D.d16 / 2; i += 256) {             // queries, then keys, four at a time

@@ -268,8 +268,8 @@ constexpr int ROUTE_LOGITS = 8192;   // logits of the choosing CTA that fit its 
 __global__ void __launch_bounds__(128) moe_route_small_kernel(const __nv_bfloat16* __restrict__ h, int64_t ldh, const __nv_bfloat16* __restrict__ router, int64_t ldr,
                                                               int B, int W, int E, int top, RouteRule rule, float* __restrict__ logits, int* __restrict__ counter,
                                                               SmallRoute R) {
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   __shared__ float part[4][SMALL_TOK];
   __shared__ float zs[ROUTE_LOGITS];
   __shared__ float gs[4][MAX_GROUPS];

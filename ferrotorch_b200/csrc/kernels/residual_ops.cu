@@ -51,8 +51,8 @@ FT_DEVICE float4 keep4(float4 v, int c, int W) {
 template <typename H>
 __global__ void __launch_bounds__(256) residual_embed_kernel(const int64_t* __restrict__ ids, const H* __restrict__ table, int64_t ld_table, int64_t vocab, float scale,
                                                              float* __restrict__ x, int64_t ldx, H* __restrict__ h, int64_t ldh, int rows, int W) {
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const int c = (blockIdx.x * 256 + threadIdx.x) * 4;
   if (c >= W) return;
   for (int r = blockIdx.y; r < rows; r += gridDim.y) {
@@ -82,8 +82,8 @@ __global__ void __launch_bounds__(TH) residual_update_kernel(float* __restrict__
     const int c = c0 + (i * TH + threadIdx.x) * 4;
     wv[i] = c < cend ? *reinterpret_cast<const float4*>(w + c) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   auto row_sum = [&](float ss, int slot) -> float {
     ss = block_sum(ss, red);
     if (ncta == 1) return ss;
@@ -187,8 +187,8 @@ __global__ void __launch_bounds__(UPD_THREADS) parallel_update_kernel(float* __r
   __shared__ float cta_ss;
   cg::cluster_group cluster = cg::this_cluster();
   const int row = blockIdx.x / ncta, c0 = blockIdx.x % ncta * cols, cend = min(W, c0 + cols);
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   float* xr = x + (size_t)row * ldx;
   int64_t id = -1;
   if constexpr (EMBED) id = ids[row];
@@ -290,8 +290,8 @@ __global__ void __launch_bounds__(TH) depth_update_kernel(DepthArgs<H> A, const 
   __shared__ float cta_ss[2];
   cg::cluster_group cluster = cg::this_cluster();
   const int row = blockIdx.x / ncta, c0 = blockIdx.x % ncta * cols, cend = min(W, c0 + cols);
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   auto row_sum = [&](float ss, int slot) -> float {
     ss = block_sum(ss, red);
     if (ncta == 1) return ss;
@@ -455,8 +455,8 @@ __global__ void __launch_bounds__(UPD_THREADS) poly_norm_kernel(const I* __restr
   __shared__ float cta_ss[3];
   cg::cluster_group cluster = cg::this_cluster();
   const int row = blockIdx.x / ncta, c0 = blockIdx.x % ncta * cols, cend = min(W, c0 + cols);
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   float4 v[NV];
   float s[3] = {0.f, 0.f, 0.f};
 #pragma unroll
@@ -592,8 +592,8 @@ __global__ void __launch_bounds__(256) gated_act_kernel(const T* __restrict__ gu
 
 __global__ void __launch_bounds__(128) gated_act_planes_kernel(const float* __restrict__ p, int splits, int64_t ldp, size_t pstride, const float* __restrict__ bias, int rows,
                                                                int quads, int kind, __nv_bfloat16* __restrict__ out, int64_t ldo) {
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const int i = blockIdx.x * 128 + threadIdx.x;
   if (i >= rows * quads) return;
   const int r = i / quads, q = i % quads;                       // four neurons

@@ -50,8 +50,8 @@ constexpr int SKINNY_U = 4;        // 32-element steps per batch of loads
 
 template <class P, int NT>
 __global__ void __launch_bounds__(256, 2) skinny_stream_kernel(const P p) {
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   extern __shared__ __align__(128) uint8_t xs[];
   __shared__ float4 red[2][8][NT][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g8 = lane >> 2, t8 = (lane & 3) * 8;

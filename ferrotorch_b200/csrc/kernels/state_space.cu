@@ -731,8 +731,8 @@ __global__ void __launch_bounds__(128) ssm_decode_conv_kernel(SsmDecode A, SsmDi
   const float4 bias = *reinterpret_cast<const float4*>(A.conv_b + (conv ? c : 0)), wl = *reinterpret_cast<const float4*>(wp + (size_t)(D.taps - 1) * cc);
   const bool zero = A.positions[b] == 0;
   float* st = A.slots + (size_t)A.slot_of[b] * A.slot_stride + D.conv_at() + (conv ? c : 0);
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const float* src = A.planes + (size_t)b * A.ldp;
   if (i < cols) {
     const float4 z = plane_sum4(src + A.z_col + i, A.splits, A.pstride);
@@ -785,8 +785,8 @@ __global__ void __launch_bounds__(256) ssm_decode_kernel(SsmDecode A, SsmDims D,
     s[i] = zero || !live || r >= D.n16 ? make_float4(0.f, 0.f, 0.f, 0.f) : *reinterpret_cast<const float4*>(S + (size_t)r * D.v16 + col);
   }
   const float skip = A.skip[hd];
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const float* u = A.u + (size_t)b * D.channels();
   for (int i = tid; i < D.n16 / 2; i += 256) {            // B, then C, four at a time
     const int r = i * 4, is_c = r >= D.n16;

@@ -59,8 +59,8 @@ template <int SM, typename H>
 __global__ void __launch_bounds__(128) hyper_update_kernel(float* __restrict__ x, int S, int64_t ldx, const float* __restrict__ mix, const float* __restrict__ out,
                                                            SubOut y, const float* __restrict__ in_next, TanhNorm norm, H* __restrict__ h, int64_t ldh, int rows,
                                                            int W, int store_x) {
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const int c = (blockIdx.x * 128 + threadIdx.x) * 4;
   if (c >= W) return;
   float cm[SM][SM], co[SM], ci[SM];
@@ -101,8 +101,8 @@ template <typename H>
 __global__ void __launch_bounds__(128) hyper_update_many_kernel(float* __restrict__ x, int S, int64_t ldx, const float* __restrict__ mix, const float* __restrict__ out,
                                                                 SubOut y, const float* __restrict__ in_next, TanhNorm norm, H* __restrict__ h, int64_t ldh, int rows,
                                                                 int W, int store_x) {
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const int c = (blockIdx.x * 128 + threadIdx.x) * 4;
   if (c >= W) return;
   const float alpha = *norm.alpha;
@@ -130,8 +130,8 @@ template <typename H>
 __global__ void __launch_bounds__(128) hyper_embed_kernel(const int64_t* __restrict__ ids, const H* __restrict__ table, int64_t ld_table, int64_t vocab,
                                                           TanhNorm first, float* __restrict__ x, int S, int64_t ldx, const float* __restrict__ in_next, TanhNorm norm,
                                                           H* __restrict__ h, int64_t ldh, int rows, int W) {
-  pdl_wait();
   pdl_launch_dependents();
+  pdl_wait();
   const int c = (blockIdx.x * 128 + threadIdx.x) * 4;
   if (c >= W) return;
   float ci = 0.f;

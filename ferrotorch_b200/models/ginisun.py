@@ -25,7 +25,7 @@ from ..errors import InvalidArgument
 from ..ops.latent_attention import (LatentDecodeBuffers, LatentDims, LatentWeights, latent_attention_decode, latent_attention_rows, rotary_pair_tables)
 from ..ops.moe import ExpertStack, MoeSmallBuffers, MoeWeights, linear_rows, moe_rows, moe_small
 from ..ops.streams import DynamicTanhWeights, HyperWeights, SublayerOutput, hyper_embed, hyper_update, round_up
-from .llama_infer import PAD_ROWS, _SplitKGemm
+from .llama_infer import PAD_ROWS, LogitsPick, _SplitKGemm
 from .registry import checked_weights
 
 EXPERT_SLOPE = 1.702          # g * sigmoid(1.702 g): fixed by the design
@@ -341,7 +341,7 @@ class GinisunModel:
                     shared[s.attn.dims] = LatentDecodeBuffers(s.attn.dims, max_batch, max_tokens, dev)
                 s.buffers = shared[s.attn.dims]
                 s.g_proj, s.g_out = _SplitKGemm(s.attn.proj, dev, planes), _SplitKGemm(s.attn.out, dev, planes)
-        self._g_head = _SplitKGemm(self.head, dev)
+        self._g_head, self._pick = _SplitKGemm(self.head, dev), LogitsPick(PAD_ROWS, dev)
         moes = [s.moe for s in self.subs if s.moe]
         self._moe_buffers = MoeSmallBuffers.allocate(moes, dev) if moes else None
         self._x = torch.zeros(PAD_ROWS, cfg.streams, self._ld, device=dev)
@@ -349,8 +349,9 @@ class GinisunModel:
         self._logits = torch.zeros(PAD_ROWS, round_up(self.vocab, 4), device=dev)[:, : self.vocab]
 
     @torch.no_grad()
-    def decode(self, state, B: int, cache) -> torch.Tensor:
-        """One token for the first ``B`` sequences of ``state``; returns the logits buffer ``[16, vocab]`` (rows below ``B`` are valid)."""
+    def decode(self, state, B: int, cache, advance: bool = False) -> torch.Tensor:
+        """One token for the first ``B`` sequences of ``state``; returns the logits buffer ``[16, vocab]`` (rows below ``B`` are valid). ``advance`` also moves ``state``
+        to the next step with the most likely tokens."""
         W, x, h = self.cfg.width, self._x, self._h
         first = self.subs[0]
         hyper_embed(state.tokens, self.embed, self.embed_norm, x, first.hyper.inp, first.norm, h, B, W)
@@ -368,5 +369,8 @@ class GinisunModel:
             hyper_update(x, s.hyper, y, None if last else nxt.hyper.inp, self.final_norm if last else nxt.norm, h, B, W, store=not last)
         self._g_head(h)
         g = self._g_head
-        _lib.call("ft_splitk_reduce", g.planes, g.splits, B, self.vocab, g.ldp, g.plane_stride, None, self._logits, self._logits.stride(0), 1, _lib.S())
+        if advance:
+            self._pick(g, self._logits, B, self.vocab, state.tokens, state.picked, state.positions, state.seq_lens)
+        else:
+            _lib.call("ft_splitk_reduce", g.planes, g.splits, B, self.vocab, g.ldp, g.plane_stride, None, self._logits, self._logits.stride(0), 1, _lib.S())
         return self._logits

@@ -56,31 +56,13 @@ class TPContext:
         return b.tensor, b.ptr_array(), b
 
 
-def _splits_for(N: int, K: int, sms: int = 148) -> int:
-    """Number of K slices for a decode GEMM. Cost model per work item (one 256-row weight tile x one K slice): weight bytes streamed,
-    32 KiB of partial-plane write + read, and ~90 KB-equivalent of pipeline fill/drain; the estimate is waves x item cost, minimised
-    over the slice counts that leave no empty slice."""
-    tiles_n = (N + 255) // 256
-    kb = (K + 63) // 64
-    best, best_t = 1, float("inf")
-    for sp in range(1, min(kb, 64) + 1):
-        kb_per = -(-kb // sp)
-        if -(-kb // kb_per) != sp:
-            continue
-        items = tiles_n * sp
-        t = math.ceil(items / sms) * (256 * kb_per * 64 * 2 + 32768 + 90000)
-        if t < best_t:
-            best, best_t = sp, t
-    return best
-
-
 class _SplitKGemm:
-    """``P[s][16][N] = x[16,K] . W[N,K]^T`` restricted to K-slice s; owns its partial-plane buffer."""
+    """``P[s][16][N] = x[16,K] . W[N,K]^T`` over ranges of K (the weight stream of a decode step); owns its partial-plane buffer."""
 
     def __init__(self, weight: torch.Tensor, device, cache: Optional[dict] = None):
         self.w = weight
         self.N, self.K = weight.shape
-        self.splits = _splits_for(self.N, self.K)
+        self.splits = _lib.kernels().ft_gemm_stream_planes(self.N, self.K)
         self.ldp = (self.N + 3) // 4 * 4
         key = (self.N, self.K)
         if cache is not None and key in cache:          # layers of the same shape share one plane buffer (they run one after another)
@@ -91,9 +73,27 @@ class _SplitKGemm:
                 cache[key] = self.planes
         self.plane_stride = PAD_ROWS * self.ldp
 
-    def __call__(self, x16: torch.Tensor) -> None:
-        _lib.call("ft_gemm_bf16_splitk", x16, self.w, self.planes, PAD_ROWS, self.N, self.K, x16.stride(0), self.w.stride(0), self.ldp, 0, 0,
-                  self.splits, _lib.S())
+    def __call__(self, x16: torch.Tensor, rows: int = PAD_ROWS) -> None:
+        """The first ``rows`` rows of ``x16``; the planes' other rows keep what they hold."""
+        _lib.call("ft_gemm_stream", x16, self.w, self.planes, rows, self.N, self.K, x16.stride(0), self.w.stride(0), self.ldp, self.splits, _lib.S())
+
+
+class LogitsPick:
+    """The end of a decode step on one rank: the head's planes summed into logits, their largest place into the next tokens, positions and lengths advanced."""
+
+    def __init__(self, rows: int, device):
+        self.rows = rows
+        self.ws = torch.zeros(rows + 1, device=device, dtype=torch.int64)
+
+    @staticmethod
+    def takes(logits: torch.Tensor) -> bool:
+        return logits.stride(0) % 4 == 0 and logits.stride(1) == 1
+
+    def __call__(self, head: _SplitKGemm, logits: torch.Tensor, rows: int, vocab: int, tokens, picked, positions, seq_lens) -> None:
+        if rows > self.rows:
+            raise InvalidArgument(f"{rows} rows, room for {self.rows}")
+        _lib.call("ft_decode_logits_pick", head.planes, head.splits, head.ldp, head.plane_stride, rows, vocab, logits, logits.stride(0), self.ws, tokens, picked,
+                  positions, seq_lens, _lib.S())
 
 
 class LlamaTPEngine:
@@ -204,6 +204,7 @@ class LlamaTPEngine:
         while d % self.ar_chunks:
             self.ar_chunks -= 1
         self.ar_sumsq = torch.zeros(2 * PAD_ROWS * self.ar_chunks, device=dev, dtype=torch.float32)
+        self.pick = LogitsPick(B, dev) if self.ctx.world == 1 and LogitsPick.takes(self.logits) else None
         # sampling exchange: every rank contributes (max logit, global index) per sequence
         self.pick_sym, self.pick_ptrs, self._pick_buf = self.ctx.symmetric(self.ctx.world * PAD_ROWS * 2, torch.float32)
         self.pick_out = torch.zeros(self.ctx.world * PAD_ROWS * 2, device=dev, dtype=torch.float32)
@@ -214,6 +215,10 @@ class LlamaTPEngine:
 
     # ------------------------------------------------------------------ pieces -------------------------------------------------------------------
     def _ar_norm(self, gemm: _SplitKGemm, w: torch.Tensor) -> None:
+        if self.ctx.world == 1 and not self.ar_cluster:
+            _lib.call("ft_decode_residual_norm", gemm.planes, gemm.splits, gemm.ldp, gemm.plane_stride, self.x, w, self.h, self.B, self.d,
+                      float(self.cfg.rms_norm_eps), _lib.S())
+            return
         if self.ar_cluster:
             _lib.call("ft_decode_ar_residual_norm_cluster", gemm.planes, gemm.splits, gemm.ldp, gemm.plane_stride,
                       self.ar_sym_push_ptrs if self.ar_push else self.ar_sym_ptrs, self.ar_flag_ptrs_cl, self.ctx.rank, self.ctx.world, self.ar_sync_cl,
@@ -288,27 +293,29 @@ class LlamaTPEngine:
 
     def _decode_body_inner(self) -> None:
         cfg, B = self.cfg, self.B
-        self.x[:B] = self.embed[self.tokens]
-        _lib.call("ft_rmsnorm_fwd", self.x, None, self.layers[0]["n1"], self.h, None, None, B, self.d, float(cfg.rms_norm_eps), _lib.S())
+        _lib.call("ft_decode_embed_norm", self.tokens, self.embed, cfg.vocab_size, self.layers[0]["n1"], self.x, self.h, B, self.d, float(cfg.rms_norm_eps), _lib.S())
         scale = 1.0 / math.sqrt(self.D)
         T = self._timed
         for li, L in enumerate(self.layers):
-            T("gemm_qkv", L["g_qkv"], self.h)
+            T("gemm_qkv", L["g_qkv"], self.h, B)
             g = L["g_qkv"]
             T("rope_kvwrite", _lib.call, "ft_decode_qkv_rope_kvwrite", g.planes, g.splits, g.ldp, g.plane_stride, B, self.Hq, self.Hkv, self.D, self.positions,
               self.cos, self.sin, self.q, self.k_cache[li], self.v_cache[li], self.block_table, self.max_blocks, _lib.S())
             T("paged_attention", _lib.call, "ft_paged_attn_decode", self.q, self.k_cache[li], self.v_cache[li], self.block_table, self.max_blocks, self.seq_lens, B,
               self.Hq, self.Hkv, self.D, float(scale), self.nsplit, self.attn_ws, self.attn_ctr, self.attn, _lib.S())
-            T("gemm_o", L["g_o"], self.attn)
+            T("gemm_o", L["g_o"], self.attn, B)
             T("allreduce_residual_norm", self._ar_norm, L["g_o"], L["n2"])
-            T("gemm_gate_up", L["g_gu"], self.h)
+            T("gemm_gate_up", L["g_gu"], self.h, B)
             g = L["g_gu"]
             T("swiglu", _lib.call, "ft_decode_swiglu", g.planes, g.splits, g.ldp, g.plane_stride, B, self.F, self.act, _lib.S())
-            T("gemm_down", L["g_d"], self.act)
+            T("gemm_down", L["g_d"], self.act, B)
             nxt = self.layers[li + 1]["n1"] if li + 1 < len(self.layers) else self.final_norm
             T("allreduce_residual_norm", self._ar_norm, L["g_d"], nxt)
-        self.g_head(self.h)
+        self.g_head(self.h, B)
         g = self.g_head
+        if self.pick is not None:
+            self.pick(g, self.logits, B, self.V, self.tokens, None, self.positions, self.seq_lens)
+            return
         _lib.call("ft_splitk_reduce", g.planes, g.splits, B, self.V, g.ldp, g.plane_stride, None, self.logits, self.V, 1, _lib.S())
         self._pick_tokens()
         self.positions += 1

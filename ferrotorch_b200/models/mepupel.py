@@ -29,7 +29,7 @@ from ..ops.residual import DenseGatedWeights, dense_gated_rows, gated_act_planes
 from ..ops.state_space import SsmDecodeBuffers, SsmDims, SsmWeights, state_space_decode, state_space_rows
 from ..ops.streams import SublayerOutput, padded_vector, round_up
 from .ginisun import ExpertConfig, MoeConfig
-from .llama_infer import PAD_ROWS, _SplitKGemm
+from .llama_infer import PAD_ROWS, LogitsPick, _SplitKGemm
 from .pufevik import AttentionConfig
 from .registry import checked_weights
 
@@ -437,7 +437,7 @@ class MepupelModel:
             if l.dense:
                 l.g_gu, l.g_down = _SplitKGemm(l.dense.gu, dev, planes.setdefault("gate", {})), _SplitKGemm(l.dense.down, dev, planes.setdefault("feed-forward", {}))
         self._side = torch.cuda.Stream(dev)
-        self._g_head = _SplitKGemm(self.head, dev)
+        self._g_head, self._pick = _SplitKGemm(self.head, dev), LogitsPick(PAD_ROWS, dev)
         moes = [l.moe for l in self.layers if l.moe]
         self._moe_buffers = MoeSmallBuffers.allocate(moes, dev) if moes else None
         self._act = {n: torch.zeros(PAD_ROWS, n, device=dev, dtype=self.dtype) for n in {l.dense.fp for l in self.layers if l.dense}}
@@ -470,8 +470,9 @@ class MepupelModel:
         return SublayerOutput(planes=l.g_down.planes, bias=d.down_bias)
 
     @torch.no_grad()
-    def decode(self, state, B: int, cache) -> torch.Tensor:
-        """One token for the first ``B`` sequences of ``state``; returns the logits buffer ``[16, vocab]`` (rows below ``B`` are valid)."""
+    def decode(self, state, B: int, cache, advance: bool = False) -> torch.Tensor:
+        """One token for the first ``B`` sequences of ``state``; returns the logits buffer ``[16, vocab]`` (rows below ``B`` are valid). ``advance`` also moves ``state``
+        to the next step with the most likely tokens."""
         cfg, W, x, h1, h2 = self.cfg, self.cfg.width, self._x, self._h1, self._h2
         parallel_embed(state.tokens, self.embed, *self._next_norms(0), cfg.eps, x, h1, h2, B)
         main, side, lib = torch.cuda.current_stream(self.device), self._side, _lib.kernels()
@@ -492,5 +493,8 @@ class MepupelModel:
             parallel_update(x, cfg.residual_mult, a, b, *self._next_norms(i + 1), cfg.eps, h1, h2, B, W, store=i + 1 < len(self.layers))
         self._g_head(h1)
         g = self._g_head
-        _lib.call("ft_splitk_reduce", g.planes, g.splits, B, self.vocab, g.ldp, g.plane_stride, None, self._logits, self._logits.stride(0), 1, _lib.S())
+        if advance:
+            self._pick(g, self._logits, B, self.vocab, state.tokens, state.picked, state.positions, state.seq_lens)
+        else:
+            _lib.call("ft_splitk_reduce", g.planes, g.splits, B, self.vocab, g.ldp, g.plane_stride, None, self._logits, self._logits.stride(0), 1, _lib.S())
         return self._logits

@@ -29,7 +29,7 @@ from ..ops.matrix_memory import MemoryDims, MemoryWeights, matrix_memory_decode,
 from ..ops.moe import linear_rows
 from ..ops.residual import DenseGatedWeights, dense_gated_rows, gated_act_planes, residual_embed, residual_update
 from ..ops.streams import SublayerOutput, padded_vector, round_up
-from .llama_infer import PAD_ROWS, _SplitKGemm
+from .llama_infer import PAD_ROWS, LogitsPick, _SplitKGemm
 from .registry import checked_weights
 
 ACTIVATION = "gelu_tanh"             # fixed by the design
@@ -452,7 +452,7 @@ class PufevikModel:
                 m.g_proj, m.g_out = _SplitKGemm(m.proj, dev, planes), _SplitKGemm(m.out, dev, planes)
             else:
                 s.g_gu, s.g_down = _SplitKGemm(s.ff.gu, dev, planes), _SplitKGemm(s.ff.down, dev, planes)
-        self._g_head = _SplitKGemm(self.head, dev)
+        self._g_head, self._pick = _SplitKGemm(self.head, dev), LogitsPick(PAD_ROWS, dev)
         ffs = [s.ff for s in self.subs if s.ff]
         self._x = torch.zeros(PAD_ROWS, self._ld, device=dev)
         self._h = torch.zeros(PAD_ROWS, self._ld, device=dev, dtype=self.dtype)[:, :W]
@@ -463,8 +463,9 @@ class PufevikModel:
         self._logits = torch.zeros(PAD_ROWS, round_up(self.vocab, 4), device=dev)[:, : self.vocab]
 
     @torch.no_grad()
-    def decode(self, state, B: int, cache) -> torch.Tensor:
-        """One token for the first ``B`` sequences of ``state``; returns the logits buffer ``[16, vocab]`` (rows below ``B`` are valid)."""
+    def decode(self, state, B: int, cache, advance: bool = False) -> torch.Tensor:
+        """One token for the first ``B`` sequences of ``state``; returns the logits buffer ``[16, vocab]`` (rows below ``B`` are valid). ``advance`` also moves ``state``
+        to the next step with the most likely tokens."""
         cfg, W, x, h = self.cfg, self.cfg.width, self._x, self._h
         mixed, act = {t.shape[1]: t for t in self._mixed}, {t.shape[1]: t for t in self._act}
         residual_embed(state.tokens, self.embed, cfg.embedding_scale, x, h, B)
@@ -472,23 +473,26 @@ class PufevikModel:
             if s.mixer:
                 m, g = s.mixer, s.mixer.g_proj
                 D, a = m.attn.dims, mixed[s.mixer.out_cols]
-                g(h)
+                g(h, B)
                 gate_col = m.main if m.memory else D.qkv_cols
                 gqa_attention_decode(g.planes, g.splits, m.attn, m.buffers, state, cache.rows[s.layer], *m.tables, B, gate_col, a[:, : D.out_cols],
                                      self._values if m.keeps_values else None, self._values if m.attn.mix is not None else None)
                 if m.memory:
                     matrix_memory_decode(g.planes, g.splits, m.memory, state, cache.states.data[s.layer], B, m.memory_col, m.memory_gate_col, a[:, D.out_cols:])
-                m.g_out(a)
+                m.g_out(a, B)
                 y = SublayerOutput(planes=m.g_out.planes)
             else:
                 a = act[s.ff.fp]
-                s.g_gu(h)
+                s.g_gu(h, B)
                 gated_act_planes(s.g_gu.planes, s.g_gu.splits, B, s.ff.fp, s.ff.act, a)
-                s.g_down(a)
+                s.g_down(a, B)
                 y = SublayerOutput(planes=s.g_down.planes)
             last = k + 1 == len(self.subs)
             residual_update(x, y, s.norm, cfg.eps, h, B, W, self.final_norm if last else None, store=not last)
-        self._g_head(h)
+        self._g_head(h, B)
         g = self._g_head
-        _lib.call("ft_splitk_reduce", g.planes, g.splits, B, self.vocab, g.ldp, g.plane_stride, None, self._logits, self._logits.stride(0), 1, _lib.S())
+        if advance:
+            self._pick(g, self._logits, B, self.vocab, state.tokens, state.picked, state.positions, state.seq_lens)
+        else:
+            _lib.call("ft_splitk_reduce", g.planes, g.splits, B, self.vocab, g.ldp, g.plane_stride, None, self._logits, self._logits.stride(0), 1, _lib.S())
         return self._logits

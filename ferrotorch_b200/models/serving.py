@@ -9,12 +9,13 @@ A model plugs in with
 * ``prepare(max_positions)``,
 * ``forward_rows(batch, cache) -> logits of batch.want``,
 * ``decode_supported()``, ``decode_begin(max_batch, max_tokens)`` and ``decode(state, batch_size, cache) -> logits`` (capturable: it reads everything that
-  changes from the state's device tensors).
+  changes from the state's device tensors); optionally ``decode(..., advance=True)``, which also leaves the most likely tokens in the state and advances it.
 
 Reference parity: ferrotorch-llama/src/generation.rs:110-404 (generation loop), ferrotorch-nn/src/paged_attention.rs:59-518 (page bookkeeping).
 """
 from __future__ import annotations
 
+import inspect
 import weakref
 from collections import deque
 from dataclasses import dataclass, field
@@ -180,6 +181,7 @@ class ServingEngine:
         self.use_graph = use_graph
         self.graphs: Dict[int, Tuple[torch.cuda.CUDAGraph, torch.Tensor]] = {}
         self.fast_decode = model.decode_supported()
+        self._advances = self.fast_decode and "advance" in inspect.signature(model.decode).parameters
         if self.fast_decode:
             self.state = DecodeState(self.device, self.max_blocks)
             model.decode_begin(DECODE_ROWS, self.max_blocks * PAGE)
@@ -282,6 +284,8 @@ class ServingEngine:
         predecessor drains and waits for it on the device)."""
         prev = _lib.kernels().ft_set_pdl(1)
         try:
+            if self._advances:
+                return self.model.decode(self.state, B, self.cache, advance=True)
             logits = self.model.decode(self.state, B, self.cache)
         finally:
             _lib.kernels().ft_set_pdl(prev)

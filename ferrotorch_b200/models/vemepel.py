@@ -31,7 +31,7 @@ from ..ops.moe import MAX_TOP, ExpertStack, MoeSmallBuffers, MoeWeights, RouteRu
 from ..ops.residual import DensePolyWeights, TokenShift, dense_poly_rows, depth_embed, depth_update, poly_norm_planes, residual_update, token_shift
 from ..ops.streams import SublayerOutput, padded_vector, round_up
 from .ginisun import MoeConfig
-from .llama_infer import PAD_ROWS, _SplitKGemm
+from .llama_infer import PAD_ROWS, LogitsPick, _SplitKGemm
 from .mepupel import DenseConfig
 from .registry import checked_weights
 
@@ -451,7 +451,7 @@ class VemepelModel:
             l.g_proj, l.g_out = _SplitKGemm(l.proj, dev, planes), _SplitKGemm(l.out, dev, planes)
             if l.dense:
                 l.g_up, l.g_down = _SplitKGemm(l.dense.up, dev, planes), _SplitKGemm(l.dense.down, dev, planes)
-        self._g_head = _SplitKGemm(self.head, dev)
+        self._g_head, self._pick = _SplitKGemm(self.head, dev), LogitsPick(PAD_ROWS, dev)
         moes = [l.moe for l in self.layers if l.moe]
         self._moe_buffers = MoeSmallBuffers.allocate(moes, dev) if moes else None
         self._act = {n: row_buffer(n) for n in {l.dense.ff for l in self.layers if l.dense}}
@@ -481,8 +481,9 @@ class VemepelModel:
         return SublayerOutput(planes=l.g_down.planes)
 
     @torch.no_grad()
-    def decode(self, state, B: int, cache) -> torch.Tensor:
-        """One token for the first ``B`` sequences of ``state``; returns the logits buffer ``[16, vocab]`` (rows below ``B`` are valid)."""
+    def decode(self, state, B: int, cache, advance: bool = False) -> torch.Tensor:
+        """One token for the first ``B`` sequences of ``state``; returns the logits buffer ``[16, vocab]`` (rows below ``B`` are valid). ``advance`` also moves ``state``
+        to the next step with the most likely tokens."""
         W, eps, x, h, results, n = self.cfg.width, self.cfg.eps, self._x, self._h, self._results, len(self.layers)
         where = dict(slots=state.slots, positions=state.positions)
         depth_embed(state.tokens, self.embed, x, results, self._next_norm(0), eps, B, h, shift=self._shift(0, cache), **where)
@@ -494,5 +495,8 @@ class VemepelModel:
             depth_update(x, results, l.average, y, w, self._next_norm(i + 1), eps, self.dtype, B, W, h, shift=self._shift(i + 1, cache), store=i + 1 < n, **where)
         self._g_head(h)
         g = self._g_head
-        _lib.call("ft_splitk_reduce", g.planes, g.splits, B, self.vocab, g.ldp, g.plane_stride, None, self._logits, self._logits.stride(0), 1, _lib.S())
+        if advance:
+            self._pick(g, self._logits, B, self.vocab, state.tokens, state.picked, state.positions, state.seq_lens)
+        else:
+            _lib.call("ft_splitk_reduce", g.planes, g.splits, B, self.vocab, g.ldp, g.plane_stride, None, self._logits, self._logits.stride(0), 1, _lib.S())
         return self._logits
