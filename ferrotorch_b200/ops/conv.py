@@ -27,6 +27,20 @@ _WGRAD_MODE = os.environ.get("FT_CONV_WGRAD", "fused")
 _ROWS_MODE = os.environ.get("FT_CONV_ROWS", "1")
 
 
+def _padded(t: torch.Tensor, top: int, left: int, bottom: int, right: int) -> torch.Tensor:
+    """``t`` ``[N, C, H, W]`` as dense ``[N, top + H + bottom, left + W + right, C]`` with zeros around every image."""
+    rows = t.permute(0, 2, 3, 1)
+    N, H, W, C = rows.shape
+    shape = (N, H + top + bottom, W + left + right, C)
+    if (t.is_cuda and t.dtype in (torch.bfloat16, torch.float16) and C % 8 == 0 and rows.is_contiguous() and t.data_ptr() % 16 == 0 and t.numel() > 0
+            and N * shape[1] * shape[2] * C // 8 < 2 ** 32 - 1024):
+        out = torch.empty(shape, device=t.device, dtype=t.dtype)
+        with _lib.on_device_of(t):
+            _lib.call("ft_pad_rows", t, out, N, H, W, C, top, left, bottom, right, _lib.S())
+        return out
+    return torch.nn.functional.pad(rows, (0, 0, left, right, top, bottom))
+
+
 def conv3x3_wgrad_gemm(x: torch.Tensor, dy: torch.Tensor) -> torch.Tensor:
     """Weight gradient of the 3x3 / stride 1 / padding 1 convolution as nine GEMMs on the tcgen05 kernel, no im2col buffer.
 
@@ -44,8 +58,8 @@ def conv3x3_wgrad_gemm(x: torch.Tensor, dy: torch.Tensor) -> torch.Tensor:
     Co = dy.shape[1]
     if dy.shape != (N, Co, H, W) or C % 8 or Co % 8:
         raise InvalidArgument("conv3x3_wgrad_gemm needs matching [N, C, H, W] tensors with channel counts that are multiples of 8")
-    xp = torch.nn.functional.pad(x.permute(0, 2, 3, 1), (0, 0, 1, 1, 1, 1)).contiguous().view(-1, C)
-    dyp = torch.nn.functional.pad(dy.permute(0, 2, 3, 1), (0, 0, 1, 1, 1, 1)).contiguous().view(-1, Co)
+    xp = _padded(x, 1, 1, 1, 1).contiguous().view(-1, C)
+    dyp = _padded(dy, 1, 1, 1, 1).contiguous().view(-1, Co)
     J = xp.shape[0]
     out = torch.empty((3, 3, Co, C), device=x.device, dtype=torch.float32)
     for r in range(3):
@@ -104,9 +118,9 @@ def conv3x3_wgrad_fused(x: torch.Tensor, dy: torch.Tensor, stride: int = 1) -> t
     Co = dy.shape[1]
     if dy.shape != (N, Co, H // stride, W // stride) or C % 64 or Co % 8 or x.dtype != torch.bfloat16 or dy.dtype != torch.bfloat16 or stride not in (1, 2):
         raise InvalidArgument("conv3x3_wgrad_fused needs bf16 [N, C, H, W] / [N, Cout, H/stride, W/stride] tensors with Cin % 64 == 0 and Cout % 8 == 0")
-    xp = torch.nn.functional.pad(x.permute(0, 2, 3, 1), (0, 0, 1, 1, 1, 1))
+    xp = _padded(x, 1, 1, 1, 1)
     if stride == 1:
-        dyp = torch.nn.functional.pad(dy.permute(0, 2, 3, 1), (0, 0, 1, 1, 1, 1)).contiguous().view(-1, Co)
+        dyp = _padded(dy, 1, 1, 1, 1).contiguous().view(-1, Co)
         shifts = [(r - 1) * (W + 2) + (s - 1) for r in range(3) for s in range(3)]
         return _wgrad_rows(dyp, xp.contiguous().view(-1, C), shifts).view(Co, 3, 3, C)
     if H % 2 or W % 2:
@@ -114,7 +128,7 @@ def conv3x3_wgrad_fused(x: torch.Tensor, dy: torch.Tensor, stride: int = 1) -> t
     Hh, Wh = (H + 2) // 2, (W + 2) // 2
     rows = N * Hh * Wh
     planes = torch.stack([xp[:, pr::2, ps::2] for pr in range(2) for ps in range(2)]).contiguous().view(4 * rows, C)
-    dyg = torch.nn.functional.pad(dy.permute(0, 2, 3, 1), (0, 0, 0, 1, 0, 1)).contiguous().view(rows, Co)           # zero last row / column
+    dyg = _padded(dy, 0, 0, 1, 1).contiguous().view(rows, Co)           # zero last row / column
     shifts = [((r % 2) * 2 + (s % 2)) * rows + (r // 2) * Wh + (s // 2) for r in range(3) for s in range(3)]
     return _wgrad_rows(dyg, planes, shifts).view(Co, 3, 3, C)
 
@@ -158,7 +172,7 @@ def conv3x3_rows(x: torch.Tensor, w_krsc: torch.Tensor, stride: int = 1, bias=No
     Co = w_krsc.shape[0]
     if w_krsc.shape != (Co, 3, 3, C) or x.dtype != torch.bfloat16 or C % 64 or Co % 8 or stride not in (1, 2):
         raise InvalidArgument("conv3x3_rows needs a bf16 [N, C, H, W] input with C % 64 == 0, [Cout, 3, 3, C] weights and stride 1 or 2")
-    xp = torch.nn.functional.pad(x.permute(0, 2, 3, 1), (0, 0, 1, 1, 1, 1))                    # [N, H+2, W+2, C]
+    xp = _padded(x, 1, 1, 1, 1)                    # [N, H+2, W+2, C]
     w3 = w_krsc.reshape(Co, 9, C)
     if stride == 1:
         Wp = W + 2
@@ -188,7 +202,7 @@ def conv3x3_dgrad_rows(dy: torch.Tensor, w_krsc: torch.Tensor, stride: int, H: i
         return conv3x3_rows(dy, w_krsc.flip(1, 2).permute(3, 1, 2, 0).contiguous(), 1)
     Hh, Wh = (H + 2) // 2, (W + 2) // 2
     rows = N * Hh * Wh
-    dyg = torch.nn.functional.pad(dy.permute(0, 2, 3, 1), (0, 0, 0, 1, 0, 1)).contiguous().view(rows, Co)
+    dyg = _padded(dy, 0, 0, 1, 1).contiguous().view(rows, Co)
     dxp = torch.empty((N, H + 2, W + 2, C), device=dy.device, dtype=torch.bfloat16)
     for pr in range(2):
         for ps in range(2):
