@@ -280,6 +280,9 @@ FT_DEVICE void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::
 // programmatic dependent launch: a kernel launched with the stream-serialization attribute may start while its predecessor is still running;
 // pdl_wait() blocks until the predecessor has completed and its writes are visible (it returns at once in an ordinary launch), and
 // pdl_launch_dependents() lets the successor's CTAs be scheduled early (they stop at their own pdl_wait).
+// The kernels of a decode step call pdl_launch_dependents() before pdl_wait(): several of them may wait on the GPU at once, each for the one before it, which in turn
+// finishes only behind its own wait. What a kernel reads ahead of its wait therefore must not be written by any kernel of the same step; the step's first kernel
+// keeps the two calls the other way round, so nothing of a step starts before the step before it is complete.
 // ---------------------------------------------------------------------------
 FT_DEVICE void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 FT_DEVICE void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -517,8 +517,9 @@ __global__ void __launch_bounds__(256) embed_norm_kernel(const int64_t* __restri
                                                          const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ h, int d, float eps,
                                                          uint32_t* status) {
   __shared__ float red[32];
-  pdl_launch_dependents();
+  // the first kernel of a step lets the next one start behind its wait: kernels that read recurrent state before their own wait must find the step before complete
   pdl_wait();
+  pdl_launch_dependents();
   const int64_t raw_id = tokens[blockIdx.x], id = raw_id < 0 ? raw_id + vocab : raw_id;
   const bool there = id >= 0 && id < vocab;
   if (!there && threadIdx.x == 0) ft_set_status(status, FT_K_PAGED, 31, blockIdx.x);

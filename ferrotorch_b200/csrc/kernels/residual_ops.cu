@@ -51,8 +51,9 @@ FT_DEVICE float4 keep4(float4 v, int c, int W) {
 template <typename H>
 __global__ void __launch_bounds__(256) residual_embed_kernel(const int64_t* __restrict__ ids, const H* __restrict__ table, int64_t ld_table, int64_t vocab, float scale,
                                                              float* __restrict__ x, int64_t ldx, H* __restrict__ h, int64_t ldh, int rows, int W) {
-  pdl_launch_dependents();
+  // the first kernel of a step lets the next one start behind its wait: kernels that read recurrent state before their own wait must find the step before complete
   pdl_wait();
+  pdl_launch_dependents();
   const int c = (blockIdx.x * 256 + threadIdx.x) * 4;
   if (c >= W) return;
   for (int r = blockIdx.y; r < rows; r += gridDim.y) {
@@ -187,8 +188,10 @@ __global__ void __launch_bounds__(UPD_THREADS) parallel_update_kernel(float* __r
   __shared__ float cta_ss;
   cg::cluster_group cluster = cg::this_cluster();
   const int row = blockIdx.x / ncta, c0 = blockIdx.x % ncta * cols, cend = min(W, c0 + cols);
-  pdl_launch_dependents();
+  // the first kernel of a step lets the next one start behind its wait: kernels that read recurrent state before their own wait must find the step before complete
+  if constexpr (!EMBED) pdl_launch_dependents();
   pdl_wait();
+  if constexpr (EMBED) pdl_launch_dependents();
   float* xr = x + (size_t)row * ldx;
   int64_t id = -1;
   if constexpr (EMBED) id = ids[row];
@@ -290,8 +293,10 @@ __global__ void __launch_bounds__(TH) depth_update_kernel(DepthArgs<H> A, const 
   __shared__ float cta_ss[2];
   cg::cluster_group cluster = cg::this_cluster();
   const int row = blockIdx.x / ncta, c0 = blockIdx.x % ncta * cols, cend = min(W, c0 + cols);
-  pdl_launch_dependents();
+  // the first kernel of a step lets the next one start behind its wait: kernels that read recurrent state before their own wait must find the step before complete
+  if constexpr (!EMBED) pdl_launch_dependents();
   pdl_wait();
+  if constexpr (EMBED) pdl_launch_dependents();
   auto row_sum = [&](float ss, int slot) -> float {
     ss = block_sum(ss, red);
     if (ncta == 1) return ss;

@@ -130,8 +130,9 @@ template <typename H>
 __global__ void __launch_bounds__(128) hyper_embed_kernel(const int64_t* __restrict__ ids, const H* __restrict__ table, int64_t ld_table, int64_t vocab,
                                                           TanhNorm first, float* __restrict__ x, int S, int64_t ldx, const float* __restrict__ in_next, TanhNorm norm,
                                                           H* __restrict__ h, int64_t ldh, int rows, int W) {
-  pdl_launch_dependents();
+  // the first kernel of a step lets the next one start behind its wait: kernels that read recurrent state before their own wait must find the step before complete
   pdl_wait();
+  pdl_launch_dependents();
   const int c = (blockIdx.x * 128 + threadIdx.x) * 4;
   if (c >= W) return;
   float ci = 0.f;
