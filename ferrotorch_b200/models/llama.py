@@ -417,7 +417,7 @@ class _EmbedFn(torch.autograd.Function):
         G = owner.acquire_grads()
         gw = G["weight"]
         if not getattr(owner, "grad_preaccumulated", False):
-            gw.zero_()
+            ops.zero_(gw)
         ops.embedding_bwd(ids, dout.reshape(-1, gw.shape[1]).contiguous(), gw)
         owner.grads_ready()
         return None, None, None

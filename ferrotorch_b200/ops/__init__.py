@@ -3,7 +3,7 @@
 from .gemm import gemm, linear, linear_master, matmul_exact, mv, dot, bmm
 from .norm import rms_norm, layer_norm, rmsnorm_fwd, rmsnorm_bwd
 from .llama import (rope_tables, rope_inplace, apply_rope, swiglu, swiglu_fwd, swiglu_bwd, embedding, embedding_fwd,
-                    embedding_bwd, scale_grads, add_)
+                    embedding_bwd, scale_grads, zero_, add_)
 from .loss import cross_entropy, cross_entropy_fwd_bwd
 from .optim import adamw_flat_, sgd_flat_, grad_norm_, scale_
 from .attention import attention_packed, flash_fwd, flash_bwd

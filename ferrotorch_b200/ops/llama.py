@@ -176,6 +176,16 @@ def embedding_fwd(ids: torch.Tensor, table: torch.Tensor) -> torch.Tensor:
     return table[flat].reshape(*ids.shape, table.shape[1])
 
 
+def zero_(t: torch.Tensor) -> torch.Tensor:
+    """Fills ``t`` with zeros."""
+    nbytes = t.numel() * t.element_size()
+    if t.is_cuda and t.is_contiguous() and nbytes % 16 == 0 and t.data_ptr() % 16 == 0 and not t.requires_grad:
+        with _lib.on_device_of(t):
+            _lib.call("ft_zero", t, nbytes, _lib.S())
+        return t
+    return t.zero_()
+
+
 def scale_grads(x: torch.Tensor, table: torch.Tensor, g: torch.Tensor) -> torch.Tensor:
     """``x * g`` as a new tensor, and ``table *= g`` in place, for a one-element ``g`` rounded to their type first."""
     if (x.is_cuda and x.dtype == table.dtype == torch.bfloat16 and g.dtype == torch.float32 and g.is_cuda and x.is_contiguous() and table.is_contiguous()

@@ -40,3 +40,10 @@ def test_scale_grads(n, m, g):
     before = x.clone()
     out = ops.scale_grads(x, table, f)
     assert torch.equal(out, want_x) and torch.equal(table, want_t) and torch.equal(x, before)
+
+
+@pytest.mark.parametrize("n", [0, 8, 8 * 1023, 8 * 1025, 8 * 70001, 12])
+def test_zero(n):
+    room = torch.full((n + 32,), 3.0, device="cuda").bfloat16()
+    ops.zero_(room[16: 16 + n])
+    assert (room[16: 16 + n] == 0).all() and (room[:16] == 3).all() and (room[16 + n:] == 3).all()
