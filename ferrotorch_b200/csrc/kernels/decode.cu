@@ -962,10 +962,10 @@ FT_EXPORT int ft_gemm_stream(const void* x, const void* w, float* planes, int ro
   if (r) return r;
   r = ft_make_tmap_2d(&tX, x, 2, true, (uint64_t)K, (uint64_t)rows, (uint64_t)ldx * 2, WS_BK, WS_TOK, CU_TENSOR_MAP_SWIZZLE_128B);
   if (r) return r;
-  static bool configured = false;
-  if (!configured) {
+  static bool configured[64] = {};
+  if (dev >= 64 || !configured[dev]) {
     FT_CUDA_TRY(cudaFuncSetAttribute(gemm_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WS_SMEM));
-    configured = true;
+    if (dev < 64) configured[dev] = true;
   }
   return (int)ft_launch_pdl(gemm_stream_kernel, dim3(ws_grid(total)), dim3(WS_THREADS), (size_t)WS_SMEM, st, tW, tX, planes, rows, N, kb, nplanes, ldp, ft_status_ptr());
 }

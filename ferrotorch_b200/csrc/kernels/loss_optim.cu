@@ -10,6 +10,7 @@
 #include "common.cuh"
 #include "host_common.h"
 #include <algorithm>
+#include <new>
 #include <vector>
 
 namespace {
@@ -448,15 +449,18 @@ int multi_update(const int64_t* rows, int count, Op op, cudaStream_t st) {
   if (count <= 0) return FT_ERR_ARG;
   for (int i = 0; i < count; i++)
     if (rows[6 * i + 5] <= 0 || !rows[6 * i] || !rows[6 * i + 4]) return FT_ERR_ARG;
-  static int resident = 0;
-  if (!resident) {
+  static const int resident = [] {
     int r = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, multi_update_kernel<GradT, Op>, 256, 0) != cudaSuccess || r < 1) r = 4;
     cudaGetLastError();
-    resident = r;
-  }
+    return r;
+  }();
   // tensors that share memory are updated one after another, in the order of the list
-  const int most = multi_disjoint(rows, count, (int)sizeof(GradT)) ? MULTI_MAX : 1;
+  int most = 1;
+  try {
+    if (multi_disjoint(rows, count, (int)sizeof(GradT))) most = MULTI_MAX;
+  } catch (const std::bad_alloc&) {                    // no memory to find out: one after another
+  }
   MultiTable t;
   for (int i = 0; i < count;) {
     uint64_t chunks = 0;
