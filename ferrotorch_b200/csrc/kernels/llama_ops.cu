@@ -168,11 +168,18 @@ __global__ void __launch_bounds__(512) embedding_bwd_scan_kernel(const int64_t* 
   const int t = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
   const int64_t id = ids[t];
   if (id < 0 || id >= vocab) return;
-  bool before = false;
-  for (int j = threadIdx.x; j < t; j += blockDim.x) before |= ids[j] == id;
+  bool before = false, later = false;                              // eight ids of a thread in flight: beside a kernel that fills the memory's queues a load takes microseconds
+#pragma unroll 8
+  for (int j = threadIdx.x; j < tokens; j += blockDim.x) {
+    const bool same = ids[j] == id;
+    before |= same && j < t;
+    later |= same && j > t;
+  }
   if (__syncthreads_or(before)) return;
-  int n = 0;                                                       // places of the id from t on, in order
-  for (int j0 = t; j0 < tokens; j0 += blockDim.x) {
+  const bool alone = !__syncthreads_or(later);
+  if (alone && threadIdx.x == 0) found[0] = (uint16_t)t;
+  int n = alone;                                                   // places of the id from t on, in order
+  for (int j0 = t; j0 < tokens && !alone; j0 += blockDim.x) {
     const int j = j0 + threadIdx.x;
     const bool mine = j < tokens && ids[j] == id;
     if (!__syncthreads_or(mine)) continue;
