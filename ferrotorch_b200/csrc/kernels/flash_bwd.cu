@@ -15,7 +15,7 @@
 // each. Every set has a score buffer; the tensor pipe works in order, so a buffer's next scores cannot pass the products that still read its P and dS. Two sets
 // (of one CTA, or of two CTAs on an SM) keep the tensor pipe from waiting for the loads, exponentials and stores of a single one.
 //
-// Bound by the chain of a step (scores, exponentials, products) more than by any pipe: the tensor pipe is about 55 % busy at 128 columns. P and dS in TMEM,
+// Bound by the chain of a step (scores, exponentials, products) more than by any pipe: the tensor pipe is 37 to 40 % busy at 128 columns, the issue slots 23 to 28 %. P and dS in TMEM,
 // two steps in flight, packed arithmetic, masks on the diagonal only, longest blocks first and the clusters: B 1, S 6001, 16 : 4 heads of 128, causal dQ 405 ->
 // 281 us, dK/dV 544 -> 373 us (790 TFLOP/s both); B 1, S 4096, 32 : 8 heads 375 -> 270 and 548 -> 334 us; heads of 64, B 32, S 197, 12 heads 58 -> 27 and
 // 68 -> 46 us.

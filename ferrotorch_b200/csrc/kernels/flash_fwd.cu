@@ -16,7 +16,7 @@
 //
 // HD is 64 or 128: a head of up to 64 columns runs at half the products and half the loads.
 //
-// Bound by the softmax warps: the exponential pipe is 55 % and the issue slots 50 % busy, the tensor pipe 50 % at 128 columns. P in TMEM instead of shared
+// Bound by the softmax warps: the exponential pipe is 55 %, the issue slots 41 to 50 % and the tensor pipe 53 % busy at 128 columns. P in TMEM instead of shared
 // memory, two f32 lanes per instruction and the longest causal blocks of all heads first: B 1, S 6001, 16 : 4 heads of 128, causal 189 -> 145 us (1020 TFLOP/s);
 // heads of 64 read in place at their own width: B 4, S 1500, 8 heads 55 us + 43 us of copies -> 43 us; B 32, S 197, 12 heads 29 us + 45 us -> 22 us.
 //
