@@ -14,6 +14,10 @@
 // V is consumed straight from its [keys, HD] row-major tile as an MN-major B operand: no transposes anywhere. The buffers of S need no release of their
 // own: the tensor pipe works in order, so S(j+2) cannot pass the O += P.V(j) that still reads its columns.
 //
+// The products O += P.V(j) complete on two barriers in turn, and every softmax warp waits for P.V(j-2) at step j: it has completed then, as S(j) runs behind it, and the
+// wait keeps the warp within one phase of each barrier. A wait by parity must never be two phases behind: it would take the phase before for the one that it means
+// (on one barrier, waited for only where O is rescaled, the end could read O ahead of the last products).
+//
 // HD is 64 or 128: a head of up to 64 columns runs at half the products and half the loads.
 //
 // Bound by the softmax warps: the exponential pipe is 55 %, the issue slots 41 to 50 % and the tensor pipe 53 % busy at 128 columns. P in TMEM instead of shared
@@ -54,10 +58,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   uint8_t* sV = sK + ST * KVB;              // ST stages
   uint64_t* bars = reinterpret_cast<uint64_t*>(sV + ST * KVB);
   uint64_t* q_full = bars + 0;
-  uint64_t* pv_done = bars + 1;
-  uint64_t* s_full = bars + 2;    // [2]
-  uint64_t* p_ready = bars + 4;   // [2]
-  uint64_t* k_full = bars + 6;    // [ST] each
+  uint64_t* pv_done = bars + 1;   // [2]
+  uint64_t* s_full = bars + 3;    // [2]
+  uint64_t* p_ready = bars + 5;   // [2]
+  uint64_t* k_full = bars + 7;    // [ST] each
   uint64_t* k_empty = k_full + ST;
   uint64_t* v_full = k_empty + ST;
   uint64_t* v_empty = v_full + ST;
@@ -77,8 +81,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
-    mbar_init(pv_done, 1);
-    for (int i = 0; i < 2; i++) { mbar_init(&s_full[i], 1); mbar_init(&p_ready[i], 4); }
+    for (int i = 0; i < 2; i++) { mbar_init(&pv_done[i], 1); mbar_init(&s_full[i], 1); mbar_init(&p_ready[i], 4); }
     for (int i = 0; i < 4 * ST; i++) mbar_init(&k_full[i], 1);
     mbar_fence_init();
   }
@@ -144,7 +147,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll
           for (int kk = 0; kk < FA_BN / 16; kk++)
             umma_f16_ts(tO, p_base + kk * 8, make_smem_desc(v_base + kk * 2048, 8192, 1024, FT_SWZ_128B), idesc_o, (j | kk) != 0);
-          umma_commit(pv_done);
+          umma_commit(&pv_done[j & 1]);
           umma_commit(&v_empty[j % ST]);
         }
       }
@@ -156,6 +159,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const uint32_t lane_off = (uint32_t)(q * 32) << 16;
     float m_used = -INFINITY, l = 0.f;
     bool ok = true;
+    auto pv = [&](int j) { return wait(&pv_done[j & 1], (j >> 1) & 1); };
     for (int j = 0; j < nblk && ok; j++) {
       if (!wait(&s_full[j & 1], (j >> 1) & 1)) { if (lane == 0) ft_set_status(status, FT_K_FA_FWD, 6, j); ok = false; break; }
       tc_fence_after();
@@ -163,7 +167,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       uint32_t sv[64];
       tmem_ld_32x32b_x32(t_s, sv);
       tmem_ld_32x32b_x32(t_s + 32, sv + 32);
+      const bool behind = j < 2 || pv(j - 2);
       tmem_ld_wait();
+      if (!behind) { if (lane == 0) ft_set_status(status, FT_K_FA_FWD, 10, j); ok = false; break; }
       const int kv0 = j * FA_BN;
       if ((causal && kv0 + FA_BN - 1 > m0) || kv0 + FA_BN > S) {
         const int last = (causal ? min(qidx, S - 1) : S - 1) - kv0;      // columns up to this one count
@@ -202,7 +208,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       l = l * alpha + ((ra.x + ra.y) + (rb.x + rb.y));
       tmem_st_32x32b_x32(t_s, pk);             // over the first half of the columns just read
       if (j > 0 && rescale) {
-        if (!wait(pv_done, (j - 1) & 1)) { if (lane == 0) ft_set_status(status, FT_K_FA_FWD, 7, j); ok = false; break; }
+        if (!pv(j - 1)) { if (lane == 0) ft_set_status(status, FT_K_FA_FWD, 7, j); ok = false; break; }
         tc_fence_after();
 #pragma unroll 1
         for (int c = 0; c < HD / 32; c++) {
@@ -217,7 +223,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       warp_arrive_after_tmem(&p_ready[j & 1]);
     }
     if (ok) {
-      if (!wait(pv_done, (nblk - 1) & 1)) { if (lane == 0) ft_set_status(status, FT_K_FA_FWD, 8, 0); ok = false; }
+      if (!pv(nblk - 1)) { if (lane == 0) ft_set_status(status, FT_K_FA_FWD, 8, 0); ok = false; }
     }
     if (ok) {
       tc_fence_after();

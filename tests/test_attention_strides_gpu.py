@@ -46,6 +46,23 @@ def test_strided_attention(B, Hq, Hkv, S, D, causal, kinds):
         assert a.shape == b.shape and (a.double() - b).norm() <= TOL * b.norm() + 2e-2 * floor
 
 
+@pytest.mark.parametrize("S", [65, 128, 129, 192, 500, 1000])
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("causal", [False, True])
+def test_scores_whose_maximum_stays(S, D, causal):
+    """Equal scores: the accumulator is never rescaled behind the first block, and the output is the mean of the values in sight. Enough heads for several waves of CTAs."""
+    if ops_backend() != "tcgen05":
+        pytest.skip("native attention kernels not built")
+    torch.manual_seed(S + D)
+    q, k = torch.zeros(4, 64, S, D, device="cuda", dtype=torch.bfloat16), torch.randn(4, 64, S, D, device="cuda").bfloat16()
+    v = torch.randn(4, 64, S, D, device="cuda").bfloat16()
+    o = nn.functional.scaled_dot_product_attention(q, k, v, is_causal=causal)
+    n = torch.arange(1, S + 1, device="cuda", dtype=torch.float64)[:, None]
+    want = v.double().cumsum(2) / n if causal else v.double().mean(2, keepdim=True).expand(4, 64, S, D)
+    # probabilities of one: the products are exact, their f32 sums are off by far less than the output's rounding of 2^-9
+    assert ((o.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-5).all()
+
+
 def ops_backend():
     from ferrotorch_b200 import ops
     return ops.attention.backend()
