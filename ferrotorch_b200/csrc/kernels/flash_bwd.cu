@@ -96,6 +96,13 @@ FT_DEVICE void p_and_ds(const uint32_t* sv, const uint32_t* dv, float scale, F n
   }
 }
 
+// Zeros at the columns outside [first, last] of 32 packed ones: a pair of query and key that does not count adds nothing whatever its score and its row's statistics are. (A score
+// of -inf instead made P NaN in a row whose own sum is not finite, and with it the gradients of values that the row does not see.)
+FT_DEVICE void keep_columns(uint32_t* packed, int first, int last) {
+#pragma unroll
+  for (int c = 0; c < 16; c++) packed[c] &= (2 * c >= first && 2 * c <= last ? 0xffffu : 0u) | (2 * c + 1 >= first && 2 * c + 1 <= last ? 0xffff0000u : 0u);
+}
+
 // ------------------------------------------------------------------------------------------------------------
 // dQ
 // ------------------------------------------------------------------------------------------------------------
@@ -232,13 +239,8 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       tmem_ld_32x32b_x32(tdP + lane_off + col, dv);
       tmem_ld_wait();
       const int kv0 = j * BN;
-      if ((causal && kv0 + BN - 1 > m0) || kv0 + BN > S) {
-        const int last = (causal ? min(qidx, S - 1) : S - 1) - kv0 - part * 32;
-#pragma unroll
-        for (int c = 0; c < 32; c++)
-          if (c > last) sv[c] = __float_as_uint(-INFINITY);
-      }
       p_and_ds(sv, dv, scale, [&](int) { return nl2; }, [&](int) { return nd2; }, nullptr, ds);
+      if ((causal && kv0 + BN - 1 > m0) || kv0 + BN > S) keep_columns(ds, 0, (causal ? min(qidx, S - 1) : S - 1) - kv0 - part * 32);
       tmem_st_32x32b_x16(tS + lane_off + col, ds);
       warp_arrive_after_tmem(&ds_ready[set]);
     }
@@ -414,14 +416,13 @@ flash_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_const
       tmem_ld_32x32b_x32(tdPt + lane_off + col, dv);
       const float* st = sStat + (it % RING) * 128 + part * 32;
       tmem_ld_wait();
-      if (causal && kv0 + BM - 1 > q0) {                    // some key of the block lies behind some query of the step
-        const int first = kv0 + r - q0 - part * 32;         // columns from this one on see the key
-#pragma unroll
-        for (int c = 0; c < 32; c++)
-          if (c < first) sv[c] = __float_as_uint(-INFINITY);
-      }
       p_and_ds(sv, dv, scale, [&](int i) { return reinterpret_cast<const ulonglong2*>(st)[i]; }, [&](int i) { return reinterpret_cast<const ulonglong2*>(st + 64)[i]; }, p,
                ds);
+      if (causal && kv0 + BM - 1 > q0) {                    // some key of the block lies behind some query of the step
+        const int first = kv0 + r - q0 - part * 32;         // columns from this one on see the key
+        keep_columns(p, first, 31);
+        keep_columns(ds, first, 31);
+      }
       tmem_st_32x32b_x16(tSt + lane_off + col, p);
       tmem_st_32x32b_x16(tdPt + lane_off + col, ds);
       warp_arrive_after_tmem(&pds_ready[set]);

@@ -63,6 +63,29 @@ def test_scores_whose_maximum_stays(S, D, causal):
     assert ((o.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-5).all()
 
 
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), float("-inf")])
+@pytest.mark.parametrize("B,Hq,Hkv,S,D,row", [(2, 2, 2, 197, 64, 70), (1, 4, 1, 300, 128, 0), (1, 2, 1, 640, 80, 129), (1, 2, 2, 100, 40, 63)])
+def test_a_query_that_is_not_finite_stays_out_of_keys_it_does_not_see(B, Hq, Hkv, S, D, row, value):
+    """Causal: the gradients of values behind query ``row``, and those of every other query, do not depend on it, so they keep their bits. (The gradients of keys are products with the
+    query itself.)"""
+    if ops_backend() != "tcgen05":
+        pytest.skip("native attention kernels not built")
+    torch.manual_seed(S + D)
+    q, k, v = (torch.randn(B, h, S, D, device="cuda").bfloat16() for h in (Hq, Hkv, Hkv))
+    g = torch.randn(B, Hq, S, D, device="cuda").bfloat16()
+    bad = q.clone()
+    bad[:, :, row] = value
+    got = []
+    for x in (q, bad):
+        leaves = [t.clone().requires_grad_() for t in (x, k, v)]
+        o = nn.functional.scaled_dot_product_attention(*leaves, is_causal=True)
+        got.append((o.detach(), *torch.autograd.grad(o, leaves, g)))
+    (o0, dq0, _, dv0), (o1, dq1, _, dv1) = got
+    others = [r for r in range(S) if r != row]
+    assert torch.equal(o0[:, :, others], o1[:, :, others]) and torch.equal(dq0[:, :, others], dq1[:, :, others])
+    assert torch.equal(dv0[:, :, row + 1:], dv1[:, :, row + 1:])
+
+
 def ops_backend():
     from ferrotorch_b200 import ops
     return ops.attention.backend()
