@@ -972,7 +972,9 @@ FT_EXPORT int ft_gemm_stream(const void* x, const void* w, float* planes, int ro
 
 // x[b] = table[tokens[b]] (bf16 [vocab, d]), h[b] = RMSNorm(x[b]) * w. d % 8 == 0, 16-byte aligned rows.
 FT_EXPORT int ft_decode_embed_norm(const int64_t* tokens, const void* table, int64_t vocab, const void* w, void* x, void* h, int rows, int d, float eps, cudaStream_t st) {
-  if (rows < 1 || d < 8 || (d & 7) || vocab < 1) return FT_ERR_ARG;
+  if (rows < 1 || d < 8 || (d & 7) || vocab < 1 || (reinterpret_cast<uintptr_t>(tokens) & 7) ||
+      ((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(h)) & 15))
+    return FT_ERR_ARG;
   return (int)ft_launch_pdl(embed_norm_kernel, dim3(rows), dim3(256), 0, st, tokens, (const __nv_bfloat16*)table, vocab, (const __nv_bfloat16*)w, (__nv_bfloat16*)x,
                             (__nv_bfloat16*)h, d, eps, ft_status_ptr());
 }
@@ -989,10 +991,12 @@ FT_EXPORT int ft_decode_logits_pick(const float* planes, int splits, int64_t ldp
                             (unsigned long long*)ws, (unsigned*)((unsigned long long*)ws + rows), tokens, picked, positions, lens);
 }
 
-// ft_decode_ar_residual_norm for a group of one rank, without staging buffers and grid barriers. d % 4 == 0.
+// ft_decode_ar_residual_norm for a group of one rank, without staging buffers and grid barriers. d % 4 == 0; planes on 16-byte, x, w and h on 8-byte boundaries.
 FT_EXPORT int ft_decode_residual_norm(const float* partial, int splits, int64_t ldp, int64_t plane_stride, void* x, const void* w, void* h, int rows, int d, float eps,
                                       cudaStream_t st) {
-  if (rows < 1 || splits < 1 || d < 4 || (d & 3) || (ldp & 3) || (plane_stride & 3)) return FT_ERR_ARG;
+  if (rows < 1 || splits < 1 || d < 4 || (d & 3) || (ldp & 3) || (plane_stride & 3) || (reinterpret_cast<uintptr_t>(partial) & 15) ||
+      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(h)) & 7))
+    return FT_ERR_ARG;
   return (int)ft_launch_pdl(residual_norm_kernel, dim3(rows * RN_CL), dim3(RN_THREADS), 0, st, partial, splits, ldp, (size_t)plane_stride, (__nv_bfloat16*)x,
                             (const __nv_bfloat16*)w, (__nv_bfloat16*)h, d, eps);
 }

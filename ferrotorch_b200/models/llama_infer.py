@@ -29,6 +29,12 @@ PAD_ROWS = 16          # decode token rows are padded to 16 (the GEMM's A-operan
 KV_BLOCK = 16
 
 
+def _dense(t: torch.Tensor) -> torch.Tensor:
+    """``t`` as dense rows from a 16-byte boundary, which is how the decode kernels read what they get by address: itself, or a copy."""
+    t = t.contiguous()
+    return t.clone() if t.data_ptr() % 16 else t
+
+
 class TPContext:
     """Rank/world of the tensor-parallel group plus the symmetric buffers the decode all-reduce uses."""
 
@@ -134,6 +140,12 @@ class LlamaTPEngine:
             g.manual_seed(seed * 1000003 + layer * 1009 + zlib.crc32(name.encode()) % 997)   # identical on every rank
             return (torch.randn(shape, device=dev, generator=g, dtype=torch.float32) * 0.02).to(torch.bfloat16)
 
+        def vector(name: str):
+            v = torch.ones(d, device=dev, dtype=torch.bfloat16) if weights is None else _dense(weights[name].to(dev, torch.bfloat16))
+            if v.numel() < d:
+                raise InvalidArgument(f"{name} has {v.numel()} elements, hidden size is {d}")
+            return v
+
         self.layers = []
         pc: dict = {}
         for i in range(cfg.num_hidden_layers):
@@ -149,12 +161,13 @@ class LlamaTPEngine:
             wgu = torch.cat([gate, up], 0).contiguous()
             del gate, up
             wd = full(p + "mlp.down_proj.weight", (d, F_t), i)[:, r * self.F:(r + 1) * self.F].contiguous()
-            n1 = weights[p + "input_layernorm.weight"].to(dev, torch.bfloat16) if weights is not None else torch.ones(d, device=dev, dtype=torch.bfloat16)
-            n2 = weights[p + "post_attention_layernorm.weight"].to(dev, torch.bfloat16) if weights is not None else torch.ones(d, device=dev, dtype=torch.bfloat16)
+            n1, n2 = vector(p + "input_layernorm.weight"), vector(p + "post_attention_layernorm.weight")
             self.layers.append(dict(wqkv=wqkv, wo=wo, wgu=wgu, wd=wd, n1=n1, n2=n2, g_qkv=_SplitKGemm(wqkv, dev, pc), g_o=_SplitKGemm(wo, dev, pc),
                                     g_gu=_SplitKGemm(wgu, dev, pc), g_d=_SplitKGemm(wd, dev, pc)))
-        self.embed = full("model.embed_tokens.weight", (cfg.vocab_size, d), 10001)
-        self.final_norm = weights["model.norm.weight"].to(dev, torch.bfloat16) if weights is not None else torch.ones(d, device=dev, dtype=torch.bfloat16)
+        self.embed = _dense(full("model.embed_tokens.weight", (cfg.vocab_size, d), 10001))
+        if self.embed.dim() != 2 or self.embed.shape[1] != d:
+            raise InvalidArgument(f"the embedding table is {tuple(self.embed.shape)}, hidden size is {d}")
+        self.final_norm = vector("model.norm.weight")
         head = self.embed if cfg.tie_word_embeddings else full("lm_head.weight", (cfg.vocab_size, d), 10002)
         self.lm_head = head[r * self.V:(r + 1) * self.V].contiguous()
         self.g_head = _SplitKGemm(self.lm_head, dev)
@@ -293,7 +306,7 @@ class LlamaTPEngine:
 
     def _decode_body_inner(self) -> None:
         cfg, B = self.cfg, self.B
-        _lib.call("ft_decode_embed_norm", self.tokens, self.embed, cfg.vocab_size, self.layers[0]["n1"], self.x, self.h, B, self.d, float(cfg.rms_norm_eps), _lib.S())
+        _lib.call("ft_decode_embed_norm", self.tokens, self.embed, self.embed.shape[0], self.layers[0]["n1"], self.x, self.h, B, self.d, float(cfg.rms_norm_eps), _lib.S())
         scale = 1.0 / math.sqrt(self.D)
         T = self._timed
         for li, L in enumerate(self.layers):

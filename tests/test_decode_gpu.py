@@ -5,6 +5,7 @@ import pytest
 import torch
 
 from ferrotorch_b200 import _lib, ops
+from ferrotorch_b200.errors import FerrotorchError, InvalidArgument
 from ferrotorch_b200.models import LlamaConfig
 from ferrotorch_b200.models.llama_infer import LlamaTPEngine, random_hf_weights, reference_last_logits
 
@@ -72,3 +73,66 @@ def test_tp_engine_single_gpu_matches_dense_reference(use_graph):
         ref = reference_last_logits(cfg, W, seq)
         assert (eng.logits - ref).abs().max().item() < 0.06 * ref.abs().max().item() + 0.02
     eng.check()
+
+
+@pytest.mark.parametrize("layout", ["transposed", "columns", "offset", "shared", "padded", "short"])
+@pytest.mark.parametrize("where", ["cuda", "cpu"])
+def test_embedding_table_in_any_layout(layout, where):
+    """The embedding table and the norm vectors as a program may hold them: prompt and decode steps read the rows of the table itself, in place or as a copy. Padded and short: more and
+    fewer rows than the vocabulary (tokens of the rows that are there)."""
+    cfg = LlamaConfig(vocab_size=512, hidden_size=256, intermediate_size=256, num_hidden_layers=1, num_attention_heads=2, num_key_value_heads=1, max_position_embeddings=64)
+    W = {k: v.to(where, torch.bfloat16) for k, v in random_hf_weights(cfg, "cuda", seed=2, std=0.05).items()}
+    e = W["model.embed_tokens.weight"]
+    V, d = e.shape
+    if layout == "transposed":
+        odd = e.t().contiguous().t()
+    elif layout == "columns":
+        odd = torch.cat([torch.full_like(e, 9.0), e], 1)[:, d:]
+    elif layout == "offset":
+        odd = torch.cat([e.new_zeros(1), e.reshape(-1)])[1:].view(V, d)
+    elif layout == "shared":
+        odd = e = e[:1].expand(V, d)
+    elif layout == "padded":
+        odd = e = torch.cat([e, e.flip(0)[:8] * 2])
+    else:
+        odd = e = e[:40]
+    plain, given = dict(W), dict(W)
+    plain["model.embed_tokens.weight"], given["model.embed_tokens.weight"] = e.contiguous(), odd
+    n = "model.layers.0.input_layernorm.weight"
+    given[n] = torch.cat([W[n][:1], W[n]])[1:]                                    # a vector from an odd place
+    engines = [LlamaTPEngine(cfg, max_batch=3, max_seq=64, device="cuda", weights=w, use_graph=False) for w in (plain, given)]
+    ids = torch.randint(0, 40, (3, 20), device="cuda", generator=torch.Generator("cuda").manual_seed(5))
+    rows = engines[0].embed.shape[0]
+    steps = torch.tensor([[0, 1, 39], [-1, -2, rows - 1], [-rows, 17, -3]], device="cuda")
+    for eng in engines:
+        eng.prefill(ids)
+    assert torch.equal(engines[0].logits, engines[1].logits)
+    full = plain["model.embed_tokens.weight"].cuda()
+    for t in steps:
+        for eng in engines:
+            eng.tokens.copy_(t)
+            eng.decode_step()
+        assert torch.equal(engines[0].logits, engines[1].logits)
+        seq = ids = torch.cat([ids, (t % rows)[:, None]], 1)
+        ref = reference_last_logits(cfg, {**plain, "model.embed_tokens.weight": full}, seq)
+        assert (engines[1].logits - ref).abs().max().item() < 0.06 * ref.abs().max().item() + 0.02
+    engines[1].check()
+
+
+def test_weights_that_do_not_fit_are_refused():
+    cfg = LlamaConfig(vocab_size=512, hidden_size=256, intermediate_size=256, num_hidden_layers=1, num_attention_heads=2, num_key_value_heads=1, max_position_embeddings=64)
+    W = random_hf_weights(cfg, "cuda", seed=2, std=0.05)
+    for name, bad in (("model.embed_tokens.weight", torch.zeros(512, 264)), ("model.norm.weight", torch.ones(128))):
+        with pytest.raises(InvalidArgument):
+            LlamaTPEngine(cfg, max_batch=1, max_seq=64, device="cuda", weights={**W, name: bad})
+
+
+def test_launchers_refuse_addresses_off_their_boundaries():
+    t = torch.zeros(4096, device="cuda", dtype=torch.bfloat16)
+    ids, planes = torch.zeros(1, device="cuda", dtype=torch.int64), torch.zeros(64, device="cuda")
+    with pytest.raises(FerrotorchError):
+        _lib.call("ft_decode_embed_norm", ids, t[1:], 4, t[1024:], t[2048:], t[3072:], 1, 64, 1e-5, _lib.S())
+    with pytest.raises(FerrotorchError):
+        _lib.call("ft_decode_residual_norm", planes[1:], 1, 4, 64, t, t[1024:], t[2048:], 1, 4, 1e-5, _lib.S())
+    with pytest.raises(FerrotorchError):
+        _lib.call("ft_decode_residual_norm", planes, 1, 4, 64, t[1:], t[1024:], t[2048:], 1, 4, 1e-5, _lib.S())
