@@ -423,14 +423,15 @@ __global__ void __launch_bounds__(256) multi_update_kernel(const __grid_constant
   }
 }
 
-// Whether no launch over these tensors could write what another of its chunks reads or writes: their address ranges are disjoint where one is written.
-bool multi_disjoint(const int64_t* rows, int count, int grad_bytes) {
+// Whether no update of these tensors writes what that of another reads or writes: their address ranges are disjoint where one is written. grad_bytes: of an element of
+// every row's gradient, or null: `same` for all.
+bool multi_disjoint(const int64_t* rows, int count, const int32_t* grad_bytes, int same) {
   struct Range { uint64_t at, end; bool written; };
   std::vector<Range> r;
   r.reserve((size_t)count * 5);
   for (int i = 0; i < count; i++) {
     const int64_t* t = rows + 6 * i;
-    const int bytes[5] = {4, 2, 4, 4, grad_bytes};
+    const int bytes[5] = {4, 2, 4, 4, grad_bytes ? grad_bytes[i] : same};
     for (int k = 0; k < 5; k++)
       if (t[k]) r.push_back({(uint64_t)t[k], (uint64_t)t[k] + (uint64_t)t[5] * bytes[k], k != 4});
   }
@@ -458,7 +459,7 @@ int multi_update(const int64_t* rows, int count, Op op, cudaStream_t st) {
   // tensors that share memory are updated one after another, in the order of the list
   int most = 1;
   try {
-    if (multi_disjoint(rows, count, (int)sizeof(GradT))) most = MULTI_MAX;
+    if (multi_disjoint(rows, count, nullptr, (int)sizeof(GradT))) most = MULTI_MAX;
   } catch (const std::bad_alloc&) {                    // no memory to find out: one after another
   }
   MultiTable t;
@@ -482,6 +483,16 @@ int multi_update(const int64_t* rows, int count, Op op, cudaStream_t st) {
   return FT_OK;
 }
 }  // namespace
+
+// 1 if the updates of these tensors (rows as below, grad_bytes: of an element of each gradient) may run in any order, 0 if some share memory that one of them writes. Host only.
+FT_EXPORT int ft_multi_disjoint(const int64_t* rows, const int32_t* grad_bytes, int count) {
+  if (count < 0) return 0;
+  try {
+    return multi_disjoint(rows, count, grad_bytes, 0) ? 1 : 0;
+  } catch (const std::bad_alloc&) {
+    return 0;
+  }
+}
 
 // AdamW over `count` tensors: rows of six 64-bit values on the host, [master f32, bf16 copy or 0, first moment, second moment, gradient, elements]. All tensors
 // are at the same step and their gradients have one type (grad_dtype: 0 = bf16, 1 = f32).

@@ -62,13 +62,21 @@ def sgd_flat_(master: torch.Tensor, p_bf16: torch.Tensor | None, buf: torch.Tens
         p_bf16.copy_(master)
 
 
+def _disjoint(runs) -> bool:
+    """Whether no tensor of these rows shares memory with another one that either update writes."""
+    rows = array.array("q", [v for _, values in runs for v in values])
+    sizes = array.array("i", [4 if f32 else 2 for (f32, _), values in runs for _ in range(len(values) // 6)])
+    return bool(_lib._fn("ft_multi_disjoint")(rows.buffer_info()[0], sizes.buffer_info()[0], len(sizes)))
+
+
 class MultiUpdate:
     """Collects the tensors of one optimizer step and updates them with a launch per kind (gradient type, step or first step) instead of one per tensor, when the block
-    ends. The tensors are held until :meth:`flush`, which launches on the stream that is current then."""
+    ends. The tensors are held until :meth:`flush`, which launches on the stream that is current then. Tensors that share memory are updated in the order of the list:
+    the launcher sees to it within a kind, :meth:`flush` across kinds."""
 
     def __init__(self, launcher: str, hyper, maximize: bool):
         self.launcher, self.hyper, self.maximize = launcher, hyper, int(maximize)
-        self.rows: dict = {}
+        self.runs: list = []                 # [kind, rows] for every stretch of the list with one kind
         self.held: list = []
 
     def __enter__(self) -> "MultiUpdate":
@@ -80,16 +88,21 @@ class MultiUpdate:
     def add(self, kind, master, low, s0, s1, grad) -> None:
         """``kind``: the step of AdamW, whether the step is the first of SGD."""
         key = (grad.dtype is torch.float32, kind)
-        rows = self.rows.get(key)
-        if rows is None:
-            rows = self.rows[key] = []
+        if not self.runs or self.runs[-1][0] != key:
+            self.runs.append((key, []))
+        rows = self.runs[-1][1]
         rows += (master.data_ptr(), 0 if low is None else low.data_ptr(), 0 if s0 is None else s0.data_ptr(), 0 if s1 is None else s1.data_ptr(), grad.data_ptr(),
                  grad.numel())
         self.held.append((master, low, s0, s1, grad))
 
     def flush(self) -> None:
-        rows, self.rows = self.rows, {}
-        for (f32, kind), values in rows.items():
+        runs, self.runs = self.runs, []
+        if len(runs) > 2 and _disjoint(runs):
+            kinds: dict = {}
+            for key, values in runs:
+                kinds.setdefault(key, []).extend(values)
+            runs = kinds.items()
+        for (f32, kind), values in runs:
             table = array.array("q", values)
             _lib.call(self.launcher, _lib.c_void_p(table.buffer_info()[0]), len(values) // 6, int(f32), *self.hyper, int(kind), self.maximize, _lib.S())
         self.held.clear()

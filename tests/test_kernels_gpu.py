@@ -205,6 +205,31 @@ def test_multi_update_matches_flat(rule, gdtype):
                 torch.testing.assert_close(a.float(), b.float(), rtol=2e-6 if a.dtype == torch.float32 else 2.0 ** -7, atol=2e-6)
 
 
+@pytest.mark.parametrize("rule", ["adamw", "sgd"])
+def test_multi_update_of_two_kinds_on_shared_memory(rule):
+    """Three updates of overlapping stretches of one master, the middle one with a gradient of another type: as if each had its own launch."""
+    from ferrotorch_b200.ops.optim import MultiUpdate
+    torch.manual_seed(3)
+    n = 5000
+    master, s0, s1 = torch.randn(n + 64, device="cuda"), torch.randn(n + 64, device="cuda"), torch.rand(n + 64, device="cuda")
+    grads = [torch.randn(n, device="cuda").to(t) for t in (torch.float32, torch.bfloat16, torch.float32)]
+    want = [t.clone() for t in (master, s0, s1)]
+    many = MultiUpdate(*(("ft_adamw_multi", (1e-2, 0.9, 0.95, 1e-8, 0.1)) if rule == "adamw" else ("ft_sgd_multi", (0.1, 0.9, 0.0, 1e-4, 1))), False)
+    with many:
+        for i, g in enumerate(grads):
+            w, a, b = (t[16 * i: 16 * i + n] for t in (master, s0, s1))
+            many.add(3 if rule == "adamw" else False, w, None, a, b if rule == "adamw" else None, g)
+    for i, g in enumerate(grads):
+        w, a, b = (t[16 * i: 16 * i + n] for t in want)
+        if rule == "adamw":
+            ops.adamw_flat_(w, None, a, b, g, lr=1e-2, beta1=0.9, beta2=0.95, eps=1e-8, weight_decay=0.1, step=3)
+        else:
+            ops.sgd_flat_(w, None, a, g, lr=0.1, momentum=0.9, weight_decay=1e-4, nesterov=True)
+    for a, b in zip((master, s0, s1), want):
+        # three updates, each within a few roundings of 2^-24 of values below ten
+        torch.testing.assert_close(a, b, rtol=6e-6, atol=6e-6)
+
+
 def test_grad_norm_and_scale():
     torch.manual_seed(9)
     a = torch.randn(100003, device="cuda")

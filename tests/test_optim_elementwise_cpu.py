@@ -91,3 +91,34 @@ def test_lbfgs_converges_like_torch(ls):
             o.step(closure)
         out.append((float(closure().detach()), w.detach().clone()))
     assert abs(out[0][0] - out[1][0]) < 1e-5 and (out[0][1] - out[1][1]).abs().max().item() < 2e-3
+
+
+@pytest.mark.parametrize("shared", ["nothing", "gradient", "master", "moment", "copy and gradient"])
+def test_updates_of_several_kinds_keep_the_order_of_the_list_where_they_share_memory(shared, monkeypatch):
+    """Kinds (gradient types, steps) take turns in a list. Tensors that share nothing, or only a gradient that both read, go out with one launch per kind; otherwise every
+    tensor goes out behind the ones ahead of it."""
+    import ctypes
+
+    from ferrotorch_b200.ops import optim as fused
+    launched = []
+    monkeypatch.setattr(fused._lib, "call", lambda name, table, count, f32, *rest: launched.append((f32, [ctypes.cast(table, ctypes.POINTER(ctypes.c_int64))[6 * i] for i in range(count)])))
+    monkeypatch.setattr(fused._lib, "S", lambda: 0)
+    rows = [[torch.zeros(40), torch.zeros(40, dtype=torch.bfloat16), torch.zeros(40), torch.zeros(40), torch.zeros(40, dtype=t)]
+            for t in (torch.float32, torch.bfloat16, torch.float32, torch.bfloat16)]
+    if shared == "gradient":
+        rows[2][4] = rows[0][4]
+    elif shared == "master":
+        room = torch.zeros(72)
+        rows[1][0], rows[2][0] = room[:40], room[32:]
+    elif shared == "moment":
+        rows[3][3] = rows[0][3]
+    elif shared == "copy and gradient":
+        rows[1][4] = rows[0][1]
+    with fused.MultiUpdate("ft_adamw_multi", (1e-3, 0.9, 0.95, 1e-8, 0.1), False) as many:
+        for r in rows:
+            many.add(1, *r)
+    at = [r[0].data_ptr() for r in rows]
+    if shared in ("nothing", "gradient"):
+        assert launched == [(1, [at[0], at[2]]), (0, [at[1], at[3]])]
+    else:
+        assert [p for _, group in launched for p in group] == at and [f for f, _ in launched] == [1, 0, 1, 0]
