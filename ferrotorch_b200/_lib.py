@@ -18,7 +18,7 @@ from pathlib import Path
 
 import torch
 
-from .errors import FerrotorchError, NativeLibraryMissing
+from .errors import FerrotorchError, IndexOutOfBounds, NativeLibraryMissing, Timeout
 
 _DIR = Path(__file__).resolve().parent / "_C"
 _lock = threading.Lock()
@@ -233,12 +233,20 @@ def call(fn_name: str, *args) -> None:
 def read_status() -> int:
     """Synchronise the current device and return (and clear) the kernel status word.
 
-    Non-zero means a bounded device-side wait ran out: bits [31:24] name the
-    kernel, [23:16] the wait site, [15:0] a detail value.
+    Non-zero means a bounded device-side wait ran out, or an index lay outside
+    its table: bits [31:24] name the kernel, [23:16] the site, [15:0] a detail
+    value (see :func:`status_error`).
     """
     out = ctypes.c_uint32(0)
     check(kernels().ft_status_read_clear(ctypes.byref(out)), "ft_status_read_clear")
     return out.value
+
+
+def status_error(st: int) -> FerrotorchError:
+    """The exception for a status word that is not zero."""
+    if st >> 24 == 0x21:
+        return IndexOutOfBounds(f"an index lies outside the table that it reads (status {st:#x})")
+    return Timeout(message=f"device-side wait timed out (status {st:#x})")
 
 
 P, S = ptr, stream_ptr          # short forms for the arguments of :func:`call`

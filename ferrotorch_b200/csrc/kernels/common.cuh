@@ -18,6 +18,7 @@
 // bit layout of a non-zero status: [31:24] kernel id, [23:16] site id, [15:0] detail
 enum FtKernelId : uint32_t {
   FT_K_GEMM = 1, FT_K_FA_FWD = 2, FT_K_FA_BWD = 3, FT_K_COMM = 4, FT_K_CONV = 5, FT_K_PAGED = 6,
+  FT_K_INDEX = 0x21,          // no wait: an index outside its table
 };
 
 FT_DEVICE void ft_set_status(uint32_t* status, uint32_t kernel, uint32_t site, uint32_t detail) {

@@ -512,17 +512,20 @@ __global__ void __launch_bounds__(128, 2) paged_attn_decode_kernel(const __nv_bf
 // ends of a decode step
 // ------------------------------------------------------------------------------------------------------------
 // x[b] = table[tokens[b]], h[b] = x[b] * rstd * w: one CTA per token, row read twice (the second time out of L1). Tokens below zero count from the table's end; one
-// outside the table reads as zeros and is reported in the status word.
+// outside the table reads as zeros and is reported in the status word and in `outside`, a word of pinned host memory that the host sees without waiting.
 __global__ void __launch_bounds__(256) embed_norm_kernel(const int64_t* __restrict__ tokens, const __nv_bfloat16* __restrict__ table, int64_t vocab,
                                                          const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ h, int d, float eps,
-                                                         uint32_t* status) {
+                                                         volatile uint32_t* outside, uint32_t* status) {
   __shared__ float red[32];
   // the first kernel of a step lets the next one start behind its wait: kernels that read recurrent state before their own wait must find the step before complete
   pdl_wait();
   pdl_launch_dependents();
   const int64_t raw_id = tokens[blockIdx.x], id = raw_id < 0 ? raw_id + vocab : raw_id;
   const bool there = id >= 0 && id < vocab;
-  if (!there && threadIdx.x == 0) ft_set_status(status, FT_K_PAGED, 31, blockIdx.x);
+  if (!there && threadIdx.x == 0) {
+    ft_set_status(status, FT_K_INDEX, 31, blockIdx.x);
+    if (outside) *outside = 1;
+  }
   const bf16x8* src = reinterpret_cast<const bf16x8*>(table + (size_t)(there ? id : 0) * d);
   bf16x8* xr = reinterpret_cast<bf16x8*>(x + (size_t)blockIdx.x * d);
   bf16x8* hr = reinterpret_cast<bf16x8*>(h + (size_t)blockIdx.x * d);
@@ -970,13 +973,18 @@ FT_EXPORT int ft_gemm_stream(const void* x, const void* w, float* planes, int ro
   return (int)ft_launch_pdl(gemm_stream_kernel, dim3(ws_grid(total)), dim3(WS_THREADS), (size_t)WS_SMEM, st, tW, tX, planes, rows, N, kb, nplanes, ldp, ft_status_ptr());
 }
 
-// x[b] = table[tokens[b]] (bf16 [vocab, d]), h[b] = RMSNorm(x[b]) * w. d % 8 == 0, 16-byte aligned rows.
-FT_EXPORT int ft_decode_embed_norm(const int64_t* tokens, const void* table, int64_t vocab, const void* w, void* x, void* h, int rows, int d, float eps, cudaStream_t st) {
+// x[b] = table[tokens[b]] (bf16 [vocab, d]), h[b] = RMSNorm(x[b]) * w. d % 8 == 0, 16-byte aligned rows. outside: null, or a word of pinned host memory that becomes 1 when a token
+// lies outside the table.
+FT_EXPORT int ft_decode_embed_norm_reporting(const int64_t* tokens, const void* table, int64_t vocab, const void* w, void* x, void* h, int rows, int d, float eps, void* outside,
+                                             cudaStream_t st) {
   if (rows < 1 || d < 8 || (d & 7) || vocab < 1 || (reinterpret_cast<uintptr_t>(tokens) & 7) ||
       ((reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(h)) & 15))
     return FT_ERR_ARG;
   return (int)ft_launch_pdl(embed_norm_kernel, dim3(rows), dim3(256), 0, st, tokens, (const __nv_bfloat16*)table, vocab, (const __nv_bfloat16*)w, (__nv_bfloat16*)x,
-                            (__nv_bfloat16*)h, d, eps, ft_status_ptr());
+                            (__nv_bfloat16*)h, d, eps, (volatile uint32_t*)outside, ft_status_ptr());
+}
+FT_EXPORT int ft_decode_embed_norm(const int64_t* tokens, const void* table, int64_t vocab, const void* w, void* x, void* h, int rows, int d, float eps, cudaStream_t st) {
+  return ft_decode_embed_norm_reporting(tokens, table, vocab, w, x, h, rows, d, eps, nullptr, st);
 }
 
 // logits[rows][ldl] = sum of the planes; tokens (and picked, if given) = place of each row's largest logit, the first of equals, a NaN before all; positions and lens

@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(256) index_select_kernel(const T* __restrict__
     int64_t s = idx[j];
     if (s < 0) s += (int64_t)src_len;
     if (s < 0 || s >= (int64_t)src_len) {
-      ft_set_status(status, 0x21, 1, (uint32_t)j);
+      ft_set_status(status, FT_K_INDEX, 1, (uint32_t)j);
       out[i] = T(0);
       continue;
     }

@@ -15,6 +15,8 @@ from __future__ import annotations
 
 import ctypes
 import math
+import threading
+import weakref
 import zlib
 from dataclasses import dataclass
 from typing import Dict, List, Optional
@@ -22,7 +24,7 @@ from typing import Dict, List, Optional
 import torch
 
 from .. import _lib, ops
-from ..errors import InvalidArgument
+from ..errors import IndexOutOfBounds, InvalidArgument
 from .llama import LlamaConfig
 
 PAD_ROWS = 16          # decode token rows are padded to 16 (the GEMM's A-operand rows)
@@ -33,6 +35,29 @@ def _dense(t: torch.Tensor) -> torch.Tensor:
     """``t`` as dense rows from a 16-byte boundary, which is how the decode kernels read what they get by address: itself, or a copy."""
     t = t.contiguous()
     return t.clone() if t.data_ptr() % 16 else t
+
+
+class _HostWords:
+    """Words of pinned host memory that a kernel sets and the host reads without waiting. The memory stays for the process; a word is given back when its owner goes, and owners
+    beyond the first thousand share one."""
+
+    def __init__(self):
+        self.lock, self.room, self.free = threading.Lock(), None, []
+
+    def take(self, owner):
+        """The word as an array of one element, and its address."""
+        with self.lock:
+            if self.room is None:
+                self.room, self.free = torch.zeros(1024, dtype=torch.int32, pin_memory=True), list(range(1, 1024))
+            at = self.free.pop() if self.free else 0
+        if at:
+            weakref.finalize(owner, self.free.append, at)
+        word = self.room.numpy()[at: at + 1]
+        word[0] = 0
+        return word, self.room.data_ptr() + 4 * at
+
+
+_host_words = _HostWords()
 
 
 class TPContext:
@@ -217,6 +242,7 @@ class LlamaTPEngine:
         while d % self.ar_chunks:
             self.ar_chunks -= 1
         self.ar_sumsq = torch.zeros(2 * PAD_ROWS * self.ar_chunks, device=dev, dtype=torch.float32)
+        self._outside, self._outside_ptr = _host_words.take(self)            # set by the step's first kernel where a token lies outside the embedding table
         self.pick = LogitsPick(B, dev) if self.ctx.world == 1 and LogitsPick.takes(self.logits) else None
         # sampling exchange: every rank contributes (max logit, global index) per sequence
         self.pick_sym, self.pick_ptrs, self._pick_buf = self.ctx.symmetric(self.ctx.world * PAD_ROWS * 2, torch.float32)
@@ -306,7 +332,8 @@ class LlamaTPEngine:
 
     def _decode_body_inner(self) -> None:
         cfg, B = self.cfg, self.B
-        _lib.call("ft_decode_embed_norm", self.tokens, self.embed, self.embed.shape[0], self.layers[0]["n1"], self.x, self.h, B, self.d, float(cfg.rms_norm_eps), _lib.S())
+        _lib.call("ft_decode_embed_norm_reporting", self.tokens, self.embed, self.embed.shape[0], self.layers[0]["n1"], self.x, self.h, B, self.d, float(cfg.rms_norm_eps),
+                  self._outside_ptr, _lib.S())
         scale = 1.0 / math.sqrt(self.D)
         T = self._timed
         for li, L in enumerate(self.layers):
@@ -342,6 +369,7 @@ class LlamaTPEngine:
         B, S = ids.shape
         if B != self.B or S + 1 > self.max_seq:
             raise InvalidArgument("prompt batch must equal the engine batch and fit the cache")
+        self._check_tokens()
         T = B * S
         x = self.embed[ids.reshape(-1).to(self.dev)]
         ar_buf = None
@@ -385,7 +413,9 @@ class LlamaTPEngine:
 
     @torch.no_grad()
     def decode_step(self) -> torch.Tensor:
-        """Feed the last sampled tokens, append their K/V, return the next tokens ``[B]`` (greedy)."""
+        """Feed the last sampled tokens, append their K/V, return the next tokens ``[B]`` (greedy). A token outside the embedding table raises at the first call behind the step that
+        met it (the host does not wait for a step), here or in :meth:`prefill`, :meth:`generate` or :meth:`check`."""
+        self._check_tokens()
         if not self.use_graph:
             self._decode_body()
             return self.tokens
@@ -414,13 +444,21 @@ class LlamaTPEngine:
         out = [self.prefill(ids)]
         for _ in range(max_new_tokens - 1):
             out.append(self.decode_step().clone())
+        if self.embed.shape[0] < self.cfg.vocab_size:          # only then can a picked token lie outside
+            torch.cuda.current_stream(self.dev).synchronize()
+            self._check_tokens()
         return torch.stack(out, 1)
+
+    def _check_tokens(self) -> None:
+        if self._outside[0]:
+            self._outside[0] = 0
+            raise IndexOutOfBounds(f"a decode step was given a token outside the embedding table of {self.embed.shape[0]} rows; its logits and the cache behind it are not those of a token")
 
     def check(self) -> None:
         st = _lib.read_status()
+        self._outside[0] = 0
         if st:
-            from ..errors import Timeout
-            raise Timeout(message=f"device-side wait timed out (status {st:#x})")
+            raise _lib.status_error(st)
 
 
 @torch.no_grad()

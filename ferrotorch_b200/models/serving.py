@@ -356,8 +356,7 @@ class ServingEngine:
     def check(self) -> None:
         st = _lib.read_status()
         if st:
-            from ..errors import Timeout
-            raise Timeout(message=f"device-side wait timed out (status {st:#x})")
+            raise _lib.status_error(st)
 
 
 @dataclass

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from ferrotorch_b200 import _lib, ops
-from ferrotorch_b200.errors import FerrotorchError, InvalidArgument
+from ferrotorch_b200.errors import FerrotorchError, IndexOutOfBounds, InvalidArgument
 from ferrotorch_b200.models import LlamaConfig
 from ferrotorch_b200.models.llama_infer import LlamaTPEngine, random_hf_weights, reference_last_logits
 
@@ -117,6 +117,33 @@ def test_embedding_table_in_any_layout(layout, where):
         ref = reference_last_logits(cfg, {**plain, "model.embed_tokens.weight": full}, seq)
         assert (engines[1].logits - ref).abs().max().item() < 0.06 * ref.abs().max().item() + 0.02
     engines[1].check()
+
+
+@pytest.mark.parametrize("use_graph", [False, True])
+def test_a_token_outside_the_table_stops_the_program(use_graph):
+    cfg = LlamaConfig(vocab_size=512, hidden_size=256, intermediate_size=256, num_hidden_layers=1, num_attention_heads=2, num_key_value_heads=1, max_position_embeddings=64)
+    W = random_hf_weights(cfg, "cuda", seed=2, std=0.05)
+    ids = torch.randint(0, 40, (2, 20), device="cuda")
+    eng, other = (LlamaTPEngine(cfg, max_batch=2, max_seq=64, device="cuda", weights=W, use_graph=use_graph) for _ in range(2))
+    for resume in (eng.decode_step, lambda: eng.prefill(ids), eng.check):
+        eng.prefill(ids)
+        other.prefill(ids)
+        eng.tokens.copy_(torch.tensor([3, 512]))
+        eng.decode_step()
+        torch.cuda.synchronize()
+        other.decode_step()                                                       # another engine goes on
+        with pytest.raises(IndexOutOfBounds, match="outside"):
+            resume()
+        assert resume == eng.check or _lib.read_status() >> 24 == 0x21
+    want = other.generate(ids, 4)
+    assert torch.equal(eng.generate(ids, 4), want)                                # and this one from its next prompt
+    eng.check()
+    few = LlamaTPEngine(cfg, max_batch=2, max_seq=64, device="cuda", weights={**W, "model.embed_tokens.weight": W["model.embed_tokens.weight"][:40]}, use_graph=use_graph)
+    assert bool((want[:, :3] >= 40).any())
+    with pytest.raises(IndexOutOfBounds):
+        few.generate(ids, 4)
+    with pytest.raises(IndexOutOfBounds):
+        few.check()
 
 
 def test_weights_that_do_not_fit_are_refused():
