@@ -187,12 +187,15 @@ def zero_(t: torch.Tensor) -> torch.Tensor:
 
 
 def scale_grads(x: torch.Tensor, table: torch.Tensor, g: torch.Tensor) -> torch.Tensor:
-    """``x * g`` as a new tensor, and ``table *= g`` in place, for a one-element ``g`` rounded to their type first."""
+    """``x * g``, and ``table *= g`` in place, for a one-element ``g`` rounded to their type first. The bf16 kernel looks at ``g`` on the device and leaves the table alone for a
+    factor of one; anything else looks at it on the host, and is given ``x`` itself then."""
     if (x.is_cuda and x.dtype == table.dtype == torch.bfloat16 and g.dtype == torch.float32 and g.is_cuda and x.is_contiguous() and table.is_contiguous()
             and x.numel() % 8 == table.numel() % 8 == 0 and x.data_ptr() % 16 == table.data_ptr() % 16 == 0):
         out = torch.empty_like(x)
         _lib.call("ft_scale_grads", x, out, x.numel(), table, table.numel(), g, _lib.S())
         return out
+    if float(g) == 1.0:
+        return x
     table.mul_(g.to(table.dtype))
     return x * g.to(x.dtype)
 

@@ -3,7 +3,7 @@ for an MLP, a transformer encoder, a CNN, an LSTM and a VAE (the same five famil
 import pytest
 import torch
 
-from ferrotorch_b200 import data, nn, optim
+from ferrotorch_b200 import data, nn, ops, optim
 
 
 def _fit(model, batches, loss_fn, opt, steps):
@@ -90,3 +90,13 @@ def test_cnn_lstm_and_vae():
         return torch.nn.functional.mse_loss(rec, target) + 1e-3 * (-0.5 * (1 + lv - mu ** 2 - lv.exp()).mean())
     first, last = _fit(vae, [(base, base)], vae_loss, optim.Adam(vae.parameters(), lr=5e-3), 200)
     assert last < 0.5 * first
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("g", [1.0, 0.5])
+def test_prepared_gradients_are_written_for_a_factor_other_than_one_only(dtype, g):
+    x, table = torch.randn(12).to(dtype), torch.randn(7, 9).to(dtype)
+    want_x, want_t, written = x * torch.tensor(g).to(dtype), table * torch.tensor(g).to(dtype), table._version
+    out = ops.scale_grads(x, table, torch.tensor(g))
+    assert torch.equal(out, want_x) and torch.equal(table, want_t)
+    assert (table._version == written) == (g == 1.0)
