@@ -224,11 +224,8 @@ int launch_conv(const void* x, const void* w, void* y, int N, int H, int W, int 
   const uint64_t yp[3] = {(uint64_t)Cout * 2, (uint64_t)W * Cout * 2, (uint64_t)H * W * Cout * 2};
   const uint32_t yb[4] = {64, PW, 4, 1};
   if ((r = ft_make_tmap_4d(&tY, y, 2, true, yd, yp, yb, CU_TENSOR_MAP_SWIZZLE_128B))) return r;
-  static bool configured = false;
-  if (!configured) {
-    FT_CUDA_TRY(cudaFuncSetAttribute(conv3x3_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM));
-    configured = true;
-  }
+  static bool configured[64] = {};
+  FT_CUDA_TRY(ft_allow_shared(conv3x3_kernel<BN>, C::SMEM, configured));
   const long long tiles = (long long)N * ((H + PH - 1) / PH) * ((W + PW - 1) / PW) * ((Cout + BN - 1) / BN);
   if (tiles > 2147483647LL) return FT_ERR_TOO_LARGE;
   const int grid = tiles < sms ? (int)tiles : sms;

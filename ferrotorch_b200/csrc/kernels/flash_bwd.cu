@@ -483,12 +483,9 @@ int launch_bwd(void* const ptr[8], const float* lse, float* stat, int B, int S, 
     const int r = make_map(m.m, ptr[m.t], B, S, m.H, D, st[m.t], m.rows);
     if (r) return r;
   }
-  static bool configured = false;
-  if (!configured) {
-    FT_CUDA_TRY(cudaFuncSetAttribute(flash_bwd_dq_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, Bwd<HD>::SMEM));
-    FT_CUDA_TRY(cudaFuncSetAttribute(flash_bwd_dkv_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, Bwd<HD>::SMEM));
-    configured = true;
-  }
+  static bool dq_configured[64] = {}, dkv_configured[64] = {};
+  FT_CUDA_TRY(ft_allow_shared(flash_bwd_dq_kernel<HD>, Bwd<HD>::SMEM, dq_configured));
+  FT_CUDA_TRY(ft_allow_shared(flash_bwd_dkv_kernel<HD>, Bwd<HD>::SMEM, dkv_configured));
   uint32_t* status = ft_status_ptr();
   const int groups = (S + 63) / 64, nm = (S + BM - 1) / BM;
   const int64_t rows = (int64_t)B * groups * 64 * Hq, units = (int64_t)nm * Hkv * B;

@@ -257,11 +257,8 @@ int launch_fwd(const void* const ptr[4], float* lse, int B, int S, int Hq, int H
     const int r = make_map(&tm[i], ptr[i], B, S, H[i], D, st[i], rows[i]);
     if (r) return r;
   }
-  static bool configured = false;
-  if (!configured) {
-    FT_CUDA_TRY(cudaFuncSetAttribute(flash_fwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, Fwd<HD>::SMEM));
-    configured = true;
-  }
+  static bool configured[64] = {};
+  FT_CUDA_TRY(ft_allow_shared(flash_fwd_kernel<HD>, Fwd<HD>::SMEM, configured));
   const int64_t ctas = (int64_t)((S + FA_BM - 1) / FA_BM) * Hq * B;
   if (ctas > 0x7fffffff) return FT_ERR_TOO_LARGE;
   flash_fwd_kernel<HD><<<(unsigned)ctas, FA_THREADS, Fwd<HD>::SMEM, stream>>>(tm[0], tm[1], tm[2], tm[3], lse, B, S, Hq, Hkv, causal, scale * LOG2E, ft_status_ptr());

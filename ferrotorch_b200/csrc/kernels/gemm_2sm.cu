@@ -387,11 +387,8 @@ template <bool A_MN, bool B_MN, bool OUT_F32>
 int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tD, const void* bias, int M, int N, int K, int k_splits, int dev,
            cudaStream_t stream, const Gemm2Epi& epi, const Gemm2Gate& gate, long long ldb_bytes) {
   auto kern = ft_gemm2_kernel<A_MN, B_MN, OUT_F32>;
-  static bool configured = false;
-  if (!configured) {
-    FT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-    configured = true;
-  }
+  static bool configured[64] = {};
+  FT_CUDA_TRY(ft_allow_shared(kern, SMEM_BYTES, configured));
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(NUM_THREADS);
   cfg.dynamicSmemBytes = SMEM_BYTES;

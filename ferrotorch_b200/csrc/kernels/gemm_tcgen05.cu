@@ -498,11 +498,8 @@ template <bool A_MN, bool B_MN, bool OUT_F32>
 int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tD, const void* bias, int M, int N, int K,
            int k_splits, int num_sms, cudaStream_t stream, const EpiArgs& epi, const TailArgs& tail) {
   auto kern = ft_gemm_kernel<A_MN, B_MN, OUT_F32>;
-  static bool configured = false;
-  if (!configured) {
-    FT_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-    configured = true;
-  }
+  static bool configured[64] = {};
+  FT_CUDA_TRY(ft_allow_shared(kern, SMEM_BYTES, configured));
   const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN) * k_splits;
   const int grid = tiles < num_sms ? tiles : num_sms;
   return (int)ft_launch_pdl(kern, dim3(grid), dim3(NUM_THREADS), (size_t)SMEM_BYTES, stream, tA, tB, tD, reinterpret_cast<const __nv_bfloat16*>(bias), M, N, K,

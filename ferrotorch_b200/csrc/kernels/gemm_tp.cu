@@ -440,11 +440,8 @@ FT_EXPORT int ft_tp_ag_gemm(const void* x_local, void* const* xg_ptrs, void* con
   if ((r = ft_make_tmap_2d(&tAg, (const __nv_bfloat16*)xg_ptrs[rank] + par_off, 2, true, (uint64_t)K, (uint64_t)M, (uint64_t)K * 2, BK, BM, CU_TENSOR_MAP_SWIZZLE_128B))) return r;
   if ((r = ft_make_tmap_2d(&tB, w_loc, 2, true, (uint64_t)K, (uint64_t)n_loc, (uint64_t)K * 2, BK, BN, CU_TENSOR_MAP_SWIZZLE_128B))) return r;
   if ((r = ft_make_tmap_2d(&tD, out, 2, true, (uint64_t)n_loc, (uint64_t)M, (uint64_t)n_loc * 2, 64, 32, CU_TENSOR_MAP_SWIZZLE_128B))) return r;
-  static bool configured = false;
-  if (!configured) {
-    FT_CUDA_TRY(cudaFuncSetAttribute(ft_tp_gemm_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-    configured = true;
-  }
+  static bool configured[64] = {};
+  FT_CUDA_TRY(ft_allow_shared(ft_tp_gemm_kernel<1>, SMEM_BYTES, configured));
   const int tiles = (M / BM) * ((n_loc + BN - 1) / BN);
   int gemm_ctas = g_sms[dev] - a.ncopy;
   if (tiles < gemm_ctas) gemm_ctas = tiles;
@@ -479,11 +476,8 @@ FT_EXPORT int ft_tp_gemm_rs(const void* x, const void* w, void* const* stage_ptr
   CUtensorMap tA, tB;
   if ((r = ft_make_tmap_2d(&tA, x, 2, true, (uint64_t)k_loc, (uint64_t)M, (uint64_t)k_loc * 2, BK, BM, CU_TENSOR_MAP_SWIZZLE_128B))) return r;
   if ((r = ft_make_tmap_2d(&tB, w, 2, true, (uint64_t)k_loc, (uint64_t)N, (uint64_t)k_loc * 2, BK, BN, CU_TENSOR_MAP_SWIZZLE_128B))) return r;
-  static bool configured = false;
-  if (!configured) {
-    FT_CUDA_TRY(cudaFuncSetAttribute(ft_tp_gemm_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-    configured = true;
-  }
+  static bool configured[64] = {};
+  FT_CUDA_TRY(ft_allow_shared(ft_tp_gemm_kernel<2>, SMEM_BYTES, configured));
   const int tiles = (M / BM) * ((N + BN - 1) / BN);
   const int grid = tiles < g_sms[dev] ? tiles : g_sms[dev];
   ft_tp_gemm_kernel<2><<<grid, NUM_THREADS, SMEM_BYTES, st>>>(tA, tA, tB, tA, sm, a, M, N, k_loc, ft_status_ptr());

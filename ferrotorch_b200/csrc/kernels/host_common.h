@@ -63,6 +63,19 @@ inline void ft_prefer_max_shared(K kernel) {
 }
 #endif
 
+// Lets `kernel` have `bytes` of dynamic shared memory on the current device. The limit belongs to a device, so it is set once on each: `done` is the launcher's static flag per device.
+#ifdef __CUDACC__
+template <typename K>
+inline cudaError_t ft_allow_shared(K kernel, int bytes, bool (&done)[64]) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess || (dev < 64 && done[dev])) return e;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess && dev < 64) done[dev] = true;
+  return e;
+}
+#endif
+
 // Launch with the programmatic-stream-serialization attribute when programmatic dependent launch is switched on (ft_set_pdl), else an ordinary
 // launch. Only kernels that call pdl_wait() before touching memory a predecessor may still be writing (or reading) go through this.
 bool ft_pdl_enabled();

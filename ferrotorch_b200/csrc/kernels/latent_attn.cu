@@ -962,11 +962,8 @@ constexpr int SMEM_MAX = 232448;
 template <int NT, int NQ, int NV>
 int launch_flash(const CUtensorMap (&m)[5], const int* tiles, int ntiles, int H, const FlashDims& F, float scale, const OutputGate& gate, void* out, int64_t ldo, int smem,
                  cudaStream_t st) {
-  static bool configured = false;
-  if (!configured) {
-    FT_CUDA_TRY(cudaFuncSetAttribute(latent_flash_kernel<NT, NQ, NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX));
-    configured = true;
-  }
+  static bool configured[64] = {};
+  FT_CUDA_TRY(ft_allow_shared(latent_flash_kernel<NT, NQ, NV>, SMEM_MAX, configured));
   latent_flash_kernel<NT, NQ, NV><<<dim3(ntiles, H), 64 + 128 * NT, smem, st>>>(m[0], m[1], m[2], m[3], m[4], reinterpret_cast<const int4*>(tiles), F,
                                                                        scale * 1.4426950408889634f, gate, (__nv_bfloat16*)out, ldo, ft_status_ptr());
   return (int)cudaGetLastError();
@@ -975,11 +972,8 @@ int launch_flash(const CUtensorMap (&m)[5], const int* tiles, int ntiles, int H,
 template <int MT, int NP>
 int launch_decode(dim3 grid, int smem, cudaStream_t st, const void* q, const void* cache, const int* bt, int mb, const int* lens, const LatentDims& D, float scale,
                   float* ws) {
-  static bool configured = false;
-  if (!configured) {
-    FT_CUDA_TRY(cudaFuncSetAttribute(latent_decode_kernel<MT, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX - 8192));
-    configured = true;
-  }
+  static bool configured[64] = {};
+  FT_CUDA_TRY(ft_allow_shared(latent_decode_kernel<MT, NP>, SMEM_MAX - 8192, configured));
   return (int)ft_launch_pdl(latent_decode_kernel<MT, NP>, grid, dim3(256), (size_t)smem, st, (const __nv_bfloat16*)q, (const __nv_bfloat16*)cache, bt, mb, lens, D, scale,
                             ws);
 }

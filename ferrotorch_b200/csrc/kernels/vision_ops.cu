@@ -68,11 +68,8 @@ FT_EXPORT int ft_nms_sorted(const float* boxes, int n, float iou_threshold, void
   if (reinterpret_cast<uintptr_t>(boxes) & 15) return FT_ERR_ARG;
   FT_CUDA_TRY(cudaMemsetAsync(mask_scratch, 0, (size_t)n * words * 8, st));
   nms_mask_kernel<<<dim3(words, words), 64, 0, st>>>((const float4*)boxes, n, iou_threshold, (unsigned long long*)mask_scratch);
-  static bool configured = false;
-  if (!configured) {
-    FT_CUDA_TRY(cudaFuncSetAttribute(nms_sweep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    configured = true;
-  }
+  static bool configured[64] = {};
+  FT_CUDA_TRY(ft_allow_shared(nms_sweep_kernel, 200 * 1024, configured));
   nms_sweep_kernel<<<1, 256, (size_t)words * 8, st>>>((const unsigned long long*)mask_scratch, n, words, (uint8_t*)keep, num_kept);
   return (int)cudaGetLastError();
 }
