@@ -139,6 +139,7 @@ gemm_stream_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       constexpr uint32_t idesc = make_idesc_f16(WS_BM, WS_TOK, 1, 0, 0);
       bool ok = true;
       int seg = 0;
+      pdl_wait();                               // the tokens come behind the kernel before: its time does not count against the limit of the waits below
       for (int64_t p = p0; p < p1 && ok; seg++) {
         const int64_t end = min(p1, (p / kblocks + 1) * kblocks);
         const int a = seg & 1;

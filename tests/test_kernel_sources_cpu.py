@@ -14,3 +14,14 @@ def test_shared_memory_limits_are_set_on_every_device(path):
     for i, line in enumerate(lines):
         if "cudaFuncAttributeMaxDynamicSharedMemorySize" in line or "ft_allow_shared(" in line:
             assert not any(re.search(r"static\s+(bool|int|cudaError_t)\s+\w+\s*=", x) for x in lines[max(0, i - 6): i]), f"{path.name}:{i + 1}"
+
+
+def test_the_weight_stream_starts_its_limits_behind_the_kernel_before():
+    """Every role of the weight stream passes the wait for the kernel before it ahead of its first bounded wait: what that kernel takes is not a wait that ran out."""
+    code = (KERNELS / "decode.cu").read_text()
+    body = code[code.index("gemm_stream_kernel(const __grid_constant__"):]
+    body = body[: body.index("\n}\n")]
+    roles = re.split(r"\n  (?:if \(warp == 0\) \{\n|\} else if \(warp == 1\) \{\n|\} else \{\n)", body)[1:]
+    assert len(roles) == 3
+    for role in roles:
+        assert 0 <= role.find("pdl_wait()") < role.index("ws_wait(")
