@@ -542,3 +542,20 @@ FT_EXPORT int ft_flash_bwd_strided(const void* q, const void* k, const void* v, 
   return D <= 64 ? launch_bwd<64>(ptr, lse, stat, B, S, Hq, Hkv, D, st, causal, scale, stream)
                  : launch_bwd<128>(ptr, lse, stat, B, S, Hq, Hkv, D, st, causal, scale, stream);
 }
+
+// The same on packed rows: qkv, dqkv: bf16 [B*S, ld]; out, dout: bf16 [B*S, Hq*128]; lse: f32 [B, Hq, S]. D must be 128. delta (f32 [B, Hq, S]) is scratch of the caller that is too
+// small for the row statistics and stays unused: they get memory of their own in the stream's order.
+FT_EXPORT int ft_flash_bwd_ws(const void* qkv, const void* out, const float* lse, const void* dout, void* dqkv, float* delta, int B, int S, int Hq, int Hkv, int D, int64_t ld,
+                              int causal, float scale, cudaStream_t stream) {
+  (void)delta;
+  if (D != 128 || B <= 0 || S <= 0 || Hq <= 0 || Hkv <= 0 || Hq % Hkv || (ld & 7)) return FT_ERR_ARG;
+  const int64_t in = (int64_t)S * ld, ldo = (int64_t)Hq * D, k = (int64_t)Hq * D, v = (int64_t)(Hq + Hkv) * D;
+  const int64_t strides[24] = {in, D, ld, in, D, ld, in, D, ld, S * ldo, D, ldo, S * ldo, D, ldo, in, D, ld, in, D, ld, in, D, ld};
+  const __nv_bfloat16* p = (const __nv_bfloat16*)qkv;
+  __nv_bfloat16* d = (__nv_bfloat16*)dqkv;
+  float* stat = nullptr;
+  FT_CUDA_TRY(cudaMallocAsync((void**)&stat, (size_t)B * Hq * ((S + 63) / 64) * 128 * sizeof(float), stream));
+  const int r = ft_flash_bwd_strided(p, p + k, p + v, out, lse, dout, d, d + k, d + v, stat, B, S, Hq, Hkv, D, strides, causal, scale, stream);
+  const cudaError_t e = cudaFreeAsync(stat, stream);
+  return r ? r : (int)e;
+}

@@ -280,3 +280,12 @@ FT_EXPORT int ft_flash_fwd_strided(const void* q, const void* k, const void* v, 
   for (int i = 0; i < 4; i++) st[i] = {strides[3 * i], strides[3 * i + 1], strides[3 * i + 2]};
   return D <= 64 ? launch_fwd<64>(ptr, lse, B, S, Hq, Hkv, D, st, causal, scale, stream) : launch_fwd<128>(ptr, lse, B, S, Hq, Hkv, D, st, causal, scale, stream);
 }
+
+// The same on the packed rows of a fused projection: qkv: bf16 [B*S, ld], the heads of q, k and v side by side; out: bf16 [B*S, Hq*128]; lse: f32 [B, Hq, S]. D must be 128.
+FT_EXPORT int ft_flash_fwd(const void* qkv, void* out, float* lse, int B, int S, int Hq, int Hkv, int D, int64_t ld, int causal, float scale, cudaStream_t stream) {
+  if (D != 128 || (ld & 7)) return FT_ERR_ARG;
+  const __nv_bfloat16* p = (const __nv_bfloat16*)qkv;
+  const int64_t in = (int64_t)S * ld, ldo = (int64_t)Hq * D;
+  const int64_t strides[12] = {in, D, ld, in, D, ld, in, D, ld, S * ldo, D, ldo};
+  return ft_flash_fwd_strided(p, p + (int64_t)Hq * D, p + (int64_t)(Hq + Hkv) * D, out, lse, B, S, Hq, Hkv, D, strides, causal, scale, stream);
+}

@@ -219,6 +219,24 @@ __global__ void __launch_bounds__(512) embedding_bwd_runs_kernel(const int64_t* 
   store_sum(acc, out);
 }
 
+// The distinct ids with the ends of their stretches of `perm`: one CTA per id.
+template <typename AccT>
+__global__ void __launch_bounds__(128) embedding_bwd_sorted_kernel(const int64_t* __restrict__ uniq_ids, const int64_t* __restrict__ seg_end, const int64_t* __restrict__ perm,
+                                                                   const __nv_bfloat16* __restrict__ dout, AccT* __restrict__ dtable, int n_uniq, int d, int64_t vocab) {
+  for (int u = blockIdx.x; u < n_uniq; u += gridDim.x) {
+    const int64_t id = uniq_ids[u];
+    if (id < 0 || id >= vocab) continue;
+    const int64_t k0 = u == 0 ? 0 : seg_end[u - 1], k1 = seg_end[u];
+    for (int c = threadIdx.x * 8; c < d; c += blockDim.x * 8) {
+      float acc[8];
+      AccT* out = dtable + (size_t)id * d + c;
+      load_sum(acc, out);
+      for (int64_t k = k0; k < k1; k++) add_row(acc, dout + (size_t)perm[k] * d + c);
+      store_sum(acc, out);
+    }
+  }
+}
+
 // out = x * g and table *= g in place, g a bf16-rounded scalar in device memory: what a loss's gradient does to the gradients that its forward pass prepared for 1.
 // A factor of 1 (every step of a training loop) leaves the table alone; it is seen here and not on the host, which does not wait for it.
 __global__ void __launch_bounds__(256) scale_grads_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ out, size_t n, __nv_bfloat16* __restrict__ table,
@@ -341,6 +359,18 @@ FT_EXPORT int ft_embedding_bwd_by_id(const int64_t* ids, const int64_t* perm, co
   else if (!perm) embedding_bwd_scan_kernel<__nv_bfloat16><<<grid, threads, 0, st>>>(ids, g, (__nv_bfloat16*)dtable, tokens, d, vocab);
   else if (acc_f32) embedding_bwd_runs_kernel<float><<<grid, threads, 0, st>>>(ids, perm, g, (float*)dtable, tokens, d, vocab);
   else embedding_bwd_runs_kernel<__nv_bfloat16><<<grid, threads, 0, st>>>(ids, perm, g, (__nv_bfloat16*)dtable, tokens, d, vocab);
+  return (int)cudaGetLastError();
+}
+
+// The same from a list of the distinct ids: uniq_ids [n_uniq] in ascending order, seg_end [n_uniq]: inclusive prefix sums of their counts, perm [tokens]: token indices sorted stably by
+// id (perm[seg_end[u-1] .. seg_end[u]) are the tokens of uniq_ids[u] in their order). d % 8 == 0.
+FT_EXPORT int ft_embedding_bwd_sorted(const int64_t* uniq_ids, const int64_t* seg_end, const int64_t* perm, const void* dout, void* dtable, int n_uniq, int d, int64_t vocab,
+                                      int acc_f32, cudaStream_t st) {
+  if (d % 8 || n_uniq <= 0) return FT_ERR_ARG;
+  const int grid = n_uniq < 148 * 16 ? n_uniq : 148 * 16;
+  const __nv_bfloat16* g = (const __nv_bfloat16*)dout;
+  if (acc_f32) embedding_bwd_sorted_kernel<float><<<grid, 128, 0, st>>>(uniq_ids, seg_end, perm, g, (float*)dtable, n_uniq, d, vocab);
+  else embedding_bwd_sorted_kernel<__nv_bfloat16><<<grid, 128, 0, st>>>(uniq_ids, seg_end, perm, g, (__nv_bfloat16*)dtable, n_uniq, d, vocab);
   return (int)cudaGetLastError();
 }
 

@@ -4,7 +4,8 @@ import math
 import pytest
 import torch
 
-from ferrotorch_b200 import ops
+from ferrotorch_b200 import _lib, ops
+from ferrotorch_b200.errors import FerrotorchError
 
 pytestmark = pytest.mark.gpu
 
@@ -94,3 +95,25 @@ def test_small_head_dims_run_on_the_padded_tcgen05_route(D, causal, Hq, Hkv, S):
     (ref * w).sum().backward()
     for a, b in ((qa, qb), (ka, kb), (va, vb)):
         assert rel(a.grad, b.grad) < 3e-2
+
+
+@pytest.mark.parametrize("B,S,Hq,Hkv,extra,causal", [(1, 1, 1, 1, 0, True), (2, 197, 4, 2, 8, False), (1, 640, 8, 1, 0, True)])
+def test_packed_launchers_of_the_c_interface(B, S, Hq, Hkv, extra, causal):
+    """``ft_flash_fwd`` and ``ft_flash_bwd_ws`` on packed rows, also of a wider buffer: the bits of the strided launchers behind ``ops``; what was refused stays refused."""
+    torch.manual_seed(S)
+    D, scale = 128, 0.1
+    n = (Hq + 2 * Hkv) * D
+    qkv = torch.randn(B * S, n + extra, device="cuda").bfloat16()
+    dout = torch.randn(B * S, Hq * D, device="cuda").bfloat16()
+    out, lse, delta = torch.empty_like(dout), torch.empty(B, Hq, S, device="cuda"), torch.empty(B, Hq, S, device="cuda")
+    dqkv = torch.zeros_like(qkv)
+    _lib.call("ft_flash_fwd", qkv, out, lse, B, S, Hq, Hkv, D, n + extra, int(causal), scale, _lib.S())
+    _lib.call("ft_flash_bwd_ws", qkv, out, lse, dout, dqkv, delta, B, S, Hq, Hkv, D, n + extra, int(causal), scale, _lib.S())
+    want, wlse = ops.flash_fwd(qkv, B, S, Hq, Hkv, D, causal, scale)
+    assert torch.equal(out, want) and torch.equal(lse, wlse)
+    assert torch.equal(dqkv[:, :n], ops.flash_bwd(qkv, want, wlse, dout, B, S, Hq, Hkv, D, causal, scale)[:, :n]) and (dqkv[:, n:] == 0).all()
+    for args in ((B, S, Hq, Hkv, 64, n + extra), (B, S, Hq, Hkv, D, n + extra + 1), (B, 0, Hq, Hkv, D, n + extra), (B, S, Hq, 3 * Hq, D, n + extra)):
+        with pytest.raises(FerrotorchError):
+            _lib.call("ft_flash_fwd", qkv, out, lse, *args, int(causal), scale, _lib.S())
+        with pytest.raises(FerrotorchError):
+            _lib.call("ft_flash_bwd_ws", qkv, out, lse, dout, dqkv, delta, *args, int(causal), scale, _lib.S())

@@ -31,6 +31,21 @@ def test_embedding_bwd_by_id(tokens, d, kind):
         assert torch.equal(got, ops.embedding_bwd(ids, dout, table.clone()))
 
 
+@pytest.mark.parametrize("tokens,d", [(1, 8), (131, 1032), (5000, 264)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_embedding_bwd_from_a_list_of_distinct_ids(tokens, d, dtype):
+    """``ft_embedding_bwd_sorted`` of the C interface: the bits of the gradient by id."""
+    torch.manual_seed(tokens + d)
+    vocab = 97
+    ids = torch.randint(-1, vocab + 1, (tokens,), device="cuda")
+    dout, table = torch.randn(tokens, d, device="cuda").bfloat16(), torch.randn(vocab, d, device="cuda").to(dtype)
+    sorted_ids, perm = torch.sort(ids, stable=True)
+    uniq, counts = torch.unique_consecutive(sorted_ids, return_counts=True)
+    got = table.clone()
+    _lib.call("ft_embedding_bwd_sorted", uniq, torch.cumsum(counts, 0), perm, dout, got, uniq.numel(), d, vocab, int(dtype == torch.float32), _lib.S())
+    assert torch.equal(got, ops.embedding_bwd(ids, dout, table.clone()))
+
+
 @pytest.mark.parametrize("g", [1.0, 0.5, 1.0001, -3.0])
 @pytest.mark.parametrize("n,m", [(8, 8), (8 * 1031, 64), (72, 8 * 70001), (12, 9)])
 def test_scale_grads(n, m, g):

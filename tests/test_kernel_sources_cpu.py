@@ -25,3 +25,10 @@ def test_the_weight_stream_starts_its_limits_behind_the_kernel_before():
     assert len(roles) == 3
     for role in roles:
         assert 0 <= role.find("pdl_wait()") < role.index("ws_wait(")
+
+
+@pytest.mark.parametrize("name", ["ft_flash_fwd", "ft_flash_bwd_ws", "ft_embedding_bwd_sorted"])
+def test_launchers_that_were_shipped_stay_in_the_c_interface(name):
+    from ferrotorch_b200 import _lib
+    header = (KERNELS.parent / "include" / "ferrotorch" / "kernels.h").read_text()
+    assert f"int {name}(" in header and hasattr(_lib.kernels(), name)
