@@ -157,6 +157,8 @@ FT_DEVICE void store_sum(const float (&acc)[8], AccT* at) {
 
 // The ids as they come: every CTA looks through all of them for its own. tokens^2 comparisons out of L2, which for up to SCAN_TOKENS tokens takes less than
 // sorting them first (a sort of 4096 ids alone takes 40 us in one CTA, and is five launches); nothing goes through the host.
+// 4096 against 4097 tokens, that is this kernel against the sort and the next one: ids at random 79 / 123 us at width 256, 38 / 140 at 1024, 57 / 164 at 4096; half of them one id 621 / 375,
+// 613 / 391, 641 / 438: what is given away there is less than what a batch without padding would lose.
 // Against the sort, the run lengths and their copy to the host before: 2331 tokens of width 1024 55 us in eight launches and a wait of the host -> 15 us in one;
 // 128 tokens of width 256 23 -> 4 us.
 constexpr int SCAN_TOKENS = 4096;
@@ -204,35 +206,73 @@ __global__ void __launch_bounds__(512) embedding_bwd_scan_kernel(const int64_t* 
   store_sum(acc, out);
 }
 
-// The ids sorted stably, with the permutation that sorted them: the first place of a run adds the run.
+// The rows of perm[k0 .. k1), in their order, 8 columns from c on per thread (none where c >= d); whole warps. A run of one id is a chain of additions, so ROWS_AHEAD rows are on their
+// way to this thread's slots (`room`, a block apart) while one is added. Copies and not loads: of loads the compiler keeps one in flight and saves the registers. A warp fetches 32 places
+// of `perm` at once: a load of the next place returns behind the rows that were requested ahead of it, and the run is a chain of round trips to memory again.
+// Half of the tokens one id, or all of them; the whole gradient, us: 16384 tokens of width 1024 1146, 2215 (with the end of the run tested between its rows 5223, 10461; the kernel over
+// distinct ids before that, one row in flight and a wait of the host, 2642, 5259); width 4096 1455, 2675 (5406, 10500; 9138, 20215). With three rows ahead 1790, 3444 at width 1024.
+constexpr int ROWS_AHEAD = 6;
+FT_DEVICE void add_rows(float (&acc)[8], const int64_t* __restrict__ perm, int64_t k0, int64_t k1, const __nv_bfloat16* __restrict__ dout, int d, int c, uint4* room) {
+  const bool on = c < d;
+  if (k1 - k0 < 3) {                                                  // most ids
+    for (int64_t k = k0; k < k1 && on; k++) add_row(acc, dout + (size_t)perm[k] * d + c);
+    return;
+  }
+  const int lane = threadIdx.x & 31;
+  for (int64_t k = k0; k < k1; k += 32) {
+    const int n = (int)min((int64_t)32, k1 - k);
+    const int64_t mine = lane < n ? perm[k + lane] : 0;
+    auto request = [&](int j, int slot) {
+      const int64_t row = __shfl_sync(0xffffffffu, mine, j & 31);
+      if (j < n && on)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(room + slot * blockDim.x)), "l"(dout + (size_t)row * d + c) : "memory");
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int j = 0; j < ROWS_AHEAD; j++) request(j, j);
+    for (int j = 0, slot = 0; j < n; j++, slot = slot + 1 < ROWS_AHEAD ? slot + 1 : 0) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(ROWS_AHEAD - 1) : "memory");
+      if (on) add_row(acc, reinterpret_cast<const __nv_bfloat16*>(room + slot * blockDim.x));
+      request(j + ROWS_AHEAD, slot);
+    }
+  }
+}
+
+// The ids sorted stably, with the permutation that sorted them: the first place of a run adds the run, whose end it looks for in steps that double and then halve (most runs are short).
 template <typename AccT>
 __global__ void __launch_bounds__(512) embedding_bwd_runs_kernel(const int64_t* __restrict__ sorted_ids, const int64_t* __restrict__ perm,
                                                                  const __nv_bfloat16* __restrict__ dout, AccT* __restrict__ dtable, int tokens, int d, int64_t vocab) {
+  extern __shared__ uint4 rows_ahead[];                               // [ROWS_AHEAD][threads]
   const int c = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
   const int t = blockIdx.x;
   const int64_t id = sorted_ids[t];
-  if (id < 0 || id >= vocab || c >= d || (t > 0 && sorted_ids[t - 1] == id)) return;
-  float acc[8];
+  if (id < 0 || id >= vocab || (t > 0 && sorted_ids[t - 1] == id)) return;
+  float acc[8] = {};
   AccT* out = dtable + (size_t)id * d + c;
-  load_sum(acc, out);
-  for (int k = t; k < tokens && sorted_ids[k] == id; k++) add_row(acc, dout + (size_t)perm[k] * d + c);
-  store_sum(acc, out);
+  if (c < d) load_sum(acc, out);
+  int64_t last = t, step = 1;                                       // sorted_ids[last] == id
+  for (; last + step < tokens && sorted_ids[last + step] == id; step *= 2) last += step;
+  for (; step > 0; step /= 2)
+    if (last + step < tokens && sorted_ids[last + step] == id) last += step;
+  add_rows(acc, perm, t, last + 1, dout, d, c, rows_ahead + threadIdx.x);
+  if (c < d) store_sum(acc, out);
 }
 
 // The distinct ids with the ends of their stretches of `perm`: one CTA per id.
 template <typename AccT>
 __global__ void __launch_bounds__(128) embedding_bwd_sorted_kernel(const int64_t* __restrict__ uniq_ids, const int64_t* __restrict__ seg_end, const int64_t* __restrict__ perm,
                                                                    const __nv_bfloat16* __restrict__ dout, AccT* __restrict__ dtable, int n_uniq, int d, int64_t vocab) {
+  __shared__ uint4 room[ROWS_AHEAD * 128];
   for (int u = blockIdx.x; u < n_uniq; u += gridDim.x) {
     const int64_t id = uniq_ids[u];
     if (id < 0 || id >= vocab) continue;
     const int64_t k0 = u == 0 ? 0 : seg_end[u - 1], k1 = seg_end[u];
-    for (int c = threadIdx.x * 8; c < d; c += blockDim.x * 8) {
-      float acc[8];
+    for (int c0 = 0; c0 < d; c0 += 128 * 8) {
+      const int c = c0 + threadIdx.x * 8;
+      float acc[8] = {};
       AccT* out = dtable + (size_t)id * d + c;
-      load_sum(acc, out);
-      for (int64_t k = k0; k < k1; k++) add_row(acc, dout + (size_t)perm[k] * d + c);
-      store_sum(acc, out);
+      if (c < d) load_sum(acc, out);
+      add_rows(acc, perm, k0, k1, dout, d, c, room + threadIdx.x);
+      if (c < d) store_sum(acc, out);
     }
   }
 }
@@ -357,8 +397,8 @@ FT_EXPORT int ft_embedding_bwd_by_id(const int64_t* ids, const int64_t* perm, co
   const __nv_bfloat16* g = (const __nv_bfloat16*)dout;
   if (!perm && acc_f32) embedding_bwd_scan_kernel<float><<<grid, threads, 0, st>>>(ids, g, (float*)dtable, tokens, d, vocab);
   else if (!perm) embedding_bwd_scan_kernel<__nv_bfloat16><<<grid, threads, 0, st>>>(ids, g, (__nv_bfloat16*)dtable, tokens, d, vocab);
-  else if (acc_f32) embedding_bwd_runs_kernel<float><<<grid, threads, 0, st>>>(ids, perm, g, (float*)dtable, tokens, d, vocab);
-  else embedding_bwd_runs_kernel<__nv_bfloat16><<<grid, threads, 0, st>>>(ids, perm, g, (__nv_bfloat16*)dtable, tokens, d, vocab);
+  else if (acc_f32) embedding_bwd_runs_kernel<float><<<grid, threads, ROWS_AHEAD * threads * 16, st>>>(ids, perm, g, (float*)dtable, tokens, d, vocab);
+  else embedding_bwd_runs_kernel<__nv_bfloat16><<<grid, threads, ROWS_AHEAD * threads * 16, st>>>(ids, perm, g, (__nv_bfloat16*)dtable, tokens, d, vocab);
   return (int)cudaGetLastError();
 }
 

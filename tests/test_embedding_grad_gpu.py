@@ -8,13 +8,16 @@ from ferrotorch_b200 import _lib, ops
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("kind", ["random", "few", "one", "outside"])
-@pytest.mark.parametrize("tokens,d", [(1, 8), (2, 4104), (131, 256), (-1, 1032), (0, 264), (1, 520), (5000, 8)])
+@pytest.mark.parametrize("kind", ["random", "few", "one", "runs", "outside"])
+@pytest.mark.parametrize("tokens,d", [(1, 8), (2, 4104), (131, 256), (-1, 1032), (0, 264), (1, 520), (5000, 8), (4500, 4104)])
 def test_embedding_bwd_by_id(tokens, d, kind):
     tokens = _lib.kernels().ft_embedding_bwd_scan_max() + tokens if tokens <= 0 or (tokens, d) == (1, 520) else tokens
     torch.manual_seed(tokens + d)
     vocab = 997
-    ids = torch.randint(0, {"random": vocab, "few": 3, "one": 1, "outside": vocab}[kind], (tokens,), device="cuda")
+    ids = torch.randint(0, {"random": vocab, "few": 3, "one": 1, "runs": vocab, "outside": vocab}[kind], (tokens,), device="cuda")
+    if kind == "runs":                                      # every length up to 98 once, in any order of the tokens
+        lengths = torch.arange(1, 100, device="cuda")
+        ids = torch.repeat_interleave(torch.arange(99, device="cuda"), lengths)[torch.randperm(4950, device="cuda")].repeat(2)[:tokens]
     if kind == "outside":
         ids[::3] = vocab
         ids[1::5] = -1
