@@ -461,7 +461,7 @@ def run_llama(size, layers, batch, prompt, ctx, steps, kernels=True):
     if kernels:
         names = {(nq, W): "qkv gemm", (W, H * 128): "output gemm", (2 * F, W): "gate/up gemm", (W, F): "down gemm"}
         roofs = {"qkv gemm": g_(nq, W), "output gemm": g_(W, H * 128), "gate/up gemm": g_(2 * F, W), "down gemm": g_(W, F),
-                 "ft_flash_fwd": (2 * T * (nq + H * 128), H * T * T * 256), "ft_rmsnorm_fwd": (6 * T * W, 0), "ft_swiglu_fwd": (6 * T * F, 0), "ft_add_bf16": (6 * T * W, 0),
+                 "ft_flash_fwd_strided": (2 * T * (nq + H * 128), H * T * T * 256), "ft_rmsnorm_fwd": (6 * T * W, 0), "ft_swiglu_fwd": (6 * T * F, 0), "ft_add_bf16": (6 * T * W, 0),
                  "ft_rope_inplace": (4 * T * (H + kvh) * 128, 0)}
         table = kernel_table(lambda: eng.prefill(ids), _by_shape(names), roofs, bw, fl)
     del eng

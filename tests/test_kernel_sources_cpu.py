@@ -32,3 +32,11 @@ def test_launchers_that_were_shipped_stay_in_the_c_interface(name):
     from ferrotorch_b200 import _lib
     header = (KERNELS.parent / "include" / "ferrotorch" / "kernels.h").read_text()
     assert f"int {name}(" in header and hasattr(_lib.kernels(), name)
+
+
+def test_benchmarks_name_launchers_that_the_package_calls():
+    """A row of a benchmark's table is keyed by the launcher's name: one that nothing calls loses its figures without a word."""
+    root = KERNELS.parents[2]
+    called = set(re.findall(r'"(ft_[a-z0-9_]+)"', "".join(p.read_text() for p in (root / "ferrotorch_b200").rglob("*.py"))))
+    named = {n for p in (root / "benchmarks").glob("*.py") for n in re.findall(r'"(ft_[a-z0-9_]+)"', p.read_text())}
+    assert named and named <= called, sorted(named - called)
