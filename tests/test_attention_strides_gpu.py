@@ -4,6 +4,7 @@ import pytest
 import torch
 
 import ferrotorch_b200.nn as nn
+from ferrotorch_b200.errors import InvalidArgument
 
 pytestmark = pytest.mark.gpu
 
@@ -97,5 +98,5 @@ def test_operands_that_do_not_fit_are_refused(refused):
     k = v = torch.zeros(1 if refused == "batch" else 2, 2, 16, 64, device="cpu" if refused == "device" else "cuda", dtype=torch.bfloat16)
     if refused == "heads":
         v = torch.zeros(2, 4, 16, 64, device="cuda", dtype=torch.bfloat16)
-    with pytest.raises(Exception):
+    with pytest.raises(InvalidArgument):
         nn.functional.scaled_dot_product_attention(q, k, v)

@@ -29,6 +29,28 @@ def test_rmsnorm_bwd(rows, d, res):
     assert torch.equal(dx, again) and torch.equal(dw, dw2)
 
 
+@pytest.mark.parametrize("d", [264, 1032, 4096, 4104])
+@pytest.mark.parametrize("where", ["x", "dy", "dres"])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+def test_rmsnorm_bwd_row_that_is_not_finite(d, where, value):
+    """One row with an element that is not finite: every other row keeps its bits, and so do the weight's gradients of columns where that row's product is unchanged (a gradient
+    element that is not finite stays in its column)."""
+    torch.manual_seed(d)
+    rows, row, col = 37, 5, 9
+    args = {n: torch.randn(rows, d, device="cuda").bfloat16() for n in ("x", "dy", "dres")}
+    w = torch.randn(d, device="cuda").bfloat16()
+    _, rstd, _ = ops.rmsnorm_fwd(args["x"], w, 1e-5)
+    got = []
+    for bad in (False, True):
+        if bad:
+            args[where][row, col] = value
+        got.append(ops.rmsnorm_bwd(args["x"], w, args["dy"], rstd, dres=args["dres"]))
+    (dx0, dw0), (dx1, dw1) = got
+    others, columns = [r for r in range(rows) if r != row], [c for c in range(d) if c != col]
+    assert torch.equal(dx0[others], dx1[others]) and not dx1[row, col].isfinite()
+    assert torch.equal(dw0[columns], dw1[columns]) and dw1[col].isfinite() == (where == "dres")
+
+
 @pytest.mark.parametrize("shape", [(1, 8, 1, 1), (2, 64, 7, 9), (3, 24, 28, 28)])
 @pytest.mark.parametrize("pads", [(1, 1, 1, 1), (0, 0, 1, 1), (2, 0, 0, 3)])
 def test_padded(shape, pads):
