@@ -1,14 +1,17 @@
 // Decode-path kernels for tensor-parallel LLM serving (small token batch, paged KV cache, block size 16).
 //
-// The projections run as split-K GEMMs (ft_gemm_bf16_splitk) that leave f32 partial planes P[s][token][n]; each kernel
+// The projections run as a weight stream (ft_gemm_stream) that leaves f32 partial planes P[s][token][n]; each kernel
 // here consumes those planes directly, summing over s on the fly, so no stand-alone reduction pass exists:
+//   ft_decode_embed_norm         a step's first kernel: embedding rows and their norm
 //   ft_decode_qkv_rope_kvwrite   sum -> RoPE at each sequence's position -> q [B,Hq,D] bf16 and K/V written into their cache pages
 //   ft_paged_attn_decode         one query token per sequence against the paged cache, GQA, split over the sequence; the last
 //                                CTA of each (sequence, kv head) merges the splits (self-resetting counters, no extra launch)
 //   ft_decode_swiglu             sum -> silu(gate)*up -> bf16
 //   ft_decode_ar_residual_norm   row-parallel output: sum of planes -> one-shot all-reduce over NVLink peer memory (fixed rank
 //                                order) -> + residual -> RMSNorm, in one kernel (the 128 KB-class all-reduce of TP decoding)
-//   ft_splitk_reduce             generic plane sum (+bias) to bf16 or f32 (LM head logits)
+//   ft_decode_residual_norm      the same on one rank
+//   ft_decode_logits_pick        a step's last kernel on one rank: logits, next tokens, positions
+//   ft_splitk_reduce             generic plane sum (+bias) to bf16 or f32 (LM head logits of several ranks)
 //   ft_paged_kv_write            copy prefill K/V rows from the packed QKV buffer into cache pages
 // Launch sequence numbers for the cross-GPU flags are read from device memory and advanced by the kernel itself, so the
 // whole decode step can be captured once in a CUDA graph and replayed.
@@ -60,7 +63,8 @@ FT_DEVICE float4 plane_sum4(const float* __restrict__ p, int splits, size_t plan
 // weights are the M side of the tensor-core tile (128 rows, 16 tokens: no work for padded rows, 16 accumulator columns). The (row tile, 64-wide k-block)
 // pairs are dealt to the CTAs in equal contiguous runs, so all of them end together; a tile that several CTAs share leaves one plane each, in the order of k,
 // and the CTA of its last k-block fills the planes that the tile does not need with zeros. Eleven 16 KiB stages per CTA; those of the first run are requested
-// before the wait for the previous kernel, which does not write weights: up to 24 MiB of them arrive behind the small kernels between two products.
+// before the wait for the previous kernel, which does not write weights: up to 148 x 11 x 16 KiB = 25.4 MiB (27 MB) of them arrive behind the small kernels between two
+// products.
 //
 // Before: 256-row tiles with 128 token rows, whole waves of equal K slices (up to 24 planes), loads behind the wait, one plane at a time in the kernels that read
 // them, seven launches for the end and the start of a step where there are two now. A prompt of 37 tokens and 24 steps of two layers of width 1024:
@@ -937,7 +941,9 @@ FT_EXPORT int ft_decode_swiglu(const float* partial, int splits, int64_t ldp, in
                             (__nv_bfloat16*)out);
 }
 
-// How many CTAs ft_gemm_stream runs on for a weight: all, unless they would have less than four k-blocks each (a plane more costs its reader as much).
+// How many CTAs ft_gemm_stream runs on for a weight: all, unless they would have less than four k-blocks each: every further CTA of a row tile is a plane more for the kernel that reads
+// them. A decode step of four layers with at least one / two / four k-blocks per CTA, us: Llama, width 1024, 1 sequence 181 / 172 / 169, 8 sequences 196 / 188 / 182; Pufevik 233 / 233 /
+// 228 and 246 / 244 / 237; width 2048: Llama 277 / 277 / 276, Pufevik 364 / 367 / 361. At width 4096 only the smallest weights are below the line: no difference.
 static int ws_grid(int64_t total) { return (int)(total < 4 * 148 ? (total + 3) / 4 : 148); }
 // Number of planes that ft_gemm_stream writes for a weight [N, K].
 FT_EXPORT int ft_gemm_stream_planes(int N, int K) {

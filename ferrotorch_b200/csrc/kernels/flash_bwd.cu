@@ -491,8 +491,10 @@ int launch_bwd(void* const ptr[8], const float* lse, float* stat, int B, int S, 
   const int64_t rows = (int64_t)B * groups * 64 * Hq, units = (int64_t)nm * Hkv * B;
   // A cluster of 1, 2 or 4 CTAs shares the query heads of a key/value head. In units of a step: a CTA takes its steps and a start and an end worth about 8 (12 in
   // a cluster of four, which adds more sums and does not fit every SM); full attention runs in whole waves, causal attention, whose blocks come longest first,
-  // until its longest CTA ends or the average SM is through. One / two / four CTAs, us of all three kernels: B 1, S 6001, 16 : 4 heads, causal 771 / 661 / 717;
-  // B 1, S 4096, 32 : 8 heads 614 / 617 / 717; B 3, S 777, 8 : 2 heads 100 / 72 / 64, full 118 / 90 / 104.
+  // until its longest CTA ends or the average SM is through. One / two / four CTAs, us of all three kernels, 128 columns: B 1, S 6001, 16 : 4 heads, causal 764 / 655 / 710; B 1, S 4096,
+  // 32 : 8 heads 608 / 611 / 713; B 3, S 777, 8 : 2 heads 94 / 65 / 57, full 111 / 82 / 97. 64 columns: 831 / 528 / 480; 632 / 461 / 459; 114 / 72 / 54, full 116 / 75 / 61; B 32, S 197,
+  // 12 : 3 heads, full 71 / 76 / 85. Over 26 shapes of both widths the choice is the fastest or within 1 % of it, but for B 1, S 8192, 8 : 2 heads of 128, causal: four, 634, where two
+  // take 588 (one 903).
   const int64_t steps = (int64_t)groups * (Hq / Hkv), slots = 148 * Bwd<HD>::CTAS;
   int ranks = 1;
   double best = 0;

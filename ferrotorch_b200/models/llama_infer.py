@@ -284,8 +284,9 @@ class LlamaTPEngine:
         self.tokens.copy_(allv[best, torch.arange(self.B, device=self.dev), 1].long())
 
     def _decode_body(self) -> None:
-        """One decode step. The step's kernels are launched as programmatic dependents (each waits on the device for its predecessor before
-        touching memory, but is scheduled while the predecessor drains), which hides the launch gaps between the ~9 small kernels of a layer.
+        """One decode step. The step's kernels are launched as programmatic dependents (each is scheduled while its predecessors run and waits on the device for the one ahead of it
+        before touching memory that a kernel of the step writes; the products request their weights ahead of that wait), which hides the launch gaps between the ~9 small kernels of
+        a layer.
         ``FT_DECODE_PDL=0`` switches to ordinary launches."""
         import os
         prev = _lib.kernels().ft_set_pdl(int(os.environ.get("FT_DECODE_PDL", "1") != "0"))
